@@ -102,7 +102,22 @@ struct dmg_fft_pass {
   int32_t *status;
   /* the tile holds more than DMG_FFT_TILE_TARGET values: the wide kernel */
   int32_t wide;
+  /* the pass runs with its lines in registers (DMG_FFT_REG_*; the tile
+   * fields above are then unused): both sides separable with the same
+   * fastest tile axis and transform-axis offsets that every line shares */
+  int32_t reg;
 };
+enum { DMG_FFT_REG_NONE = 0, DMG_FFT_REG_V1 = 1, DMG_FFT_REG_T = 2 };
+
+/* lengths with a register schedule, for values of es bytes */
+static inline int dmg_fft_reg_length(int n, int es) {
+  switch (n) {
+    case 32: case 48: case 64: case 96: case 120: case 128: case 160: case 192: case 240: case 256: case 320:
+    case 384: case 480: case 512: case 1024: return 1;
+    case 2048: return es == 8;
+    default: return 0;
+  }
+}
 
 /* Threads per pass block; the most values a tile may hold, and the number
  * the planner aims at (32 KB per tile buffer) for a value of es bytes. */

@@ -94,7 +94,7 @@ struct dmg_split_impl {
   int timing;
   void *events;
   int timed_dir, timed_passes, collected;
-  char desc[768];
+  char desc[896];
 };
 
 /* timing helpers live in the CUDA runtime source */
@@ -482,6 +482,38 @@ static int t0_rel32(const fft_layout *l, const struct dmg_fft_pass *p) {
   return 1;
 }
 
+/* whether every line of a pass shares a side's offsets along the transform
+ * axis (the table's differences from each line's first entry), as int32 */
+static int line_offsets32(const fft_layout *l, const struct dmg_fft_pass *p) {
+  if (l->ranked) return 0;
+  const int d = p->kdim[0], z = p->kisz[0];
+  const int step = z ? p->A[d] : 1;             /* coordinate step along the line */
+  const int starts = z ? p->A[d] : p->B[d];     /* lines of that dimension ... */
+  const int between = z ? 1 : p->A[d];          /* ... and the distance of their first coordinates */
+  const int64_t *t = l->tab[d];
+  for (int i = 0; i < p->n; ++i) {
+    const int64_t v = t[(int64_t)i * step] - t[0];
+    if (v < INT32_MIN || v > INT32_MAX) return 0;
+    for (int s = 1; s < starts; ++s)
+      if (t[(int64_t)s * between + (int64_t)i * step] - t[(int64_t)s * between] != v) return 0;
+  }
+  return 1;
+}
+
+/* The form in which a pass runs with its lines in registers: along t or
+ * along v1, whichever is fastest in memory on both sides.  Passes with a
+ * tile size or radix schedule of the caller's, ranked sides, or different
+ * fastest axes stay with the tiled kernel. */
+static int reg_form(const struct dmg_split_impl *im, const struct dmg_fft_pass *p, const fft_layout *li,
+                    const fft_layout *lo) {
+  if (im->tile_values > 0 || p->radix_runtime || !dmg_fft_reg_length(p->n, im->esize)) return DMG_FFT_REG_NONE;
+  if (im->arith == DMG_ARITH_TC16 && p->n == 1024) return DMG_FFT_REG_NONE;
+  if (p->sign < 0 ? p->perm_in : p->perm_out) return DMG_FFT_REG_NONE;
+  if (p->load_order[0] != p->store_order[0] || p->load_order[0] == 2) return DMG_FFT_REG_NONE;
+  if (!line_offsets32(li, p) || !line_offsets32(lo, p)) return DMG_FFT_REG_NONE;
+  return p->load_order[0] == 0 ? DMG_FFT_REG_T : DMG_FFT_REG_V1;
+}
+
 static void fill_side(struct dmg_fft_layout *fl, const fft_layout *hl, int nd, int64_t base) {
   memset(fl, 0, sizeof(*fl));
   for (int d = 0; d < nd; ++d) {
@@ -633,19 +665,24 @@ static int impl_upload(struct dmg_split_impl *im) {
       fill_side(&list[k].p.out, &im->lay[list[k].out_lay], nd, list[k].out_base);
       list[k].p.t0_rel_in = list[k].p.sep_in && t0_rel32(&im->lay[list[k].in_lay], &list[k].p);
       list[k].p.t0_rel_out = list[k].p.sep_out && t0_rel32(&im->lay[list[k].out_lay], &list[k].p);
+      const fft_layout *li = &im->lay[list[k].in_lay], *lo = &im->lay[list[k].out_lay];
+      list[k].p.reg = reg_form(im, &list[k].p, li, lo);
       /* scratch variant: an upper-half side moves to the fixed array */
       pass_rec *sr = dir == 0 ? &im->fwd_s[k] : &im->inv_s[k];
       *sr = list[k];
       if (sr->in_buf == BUF_WORK && sr->in_base != 0) {
         sr->in_buf = BUF_SCRATCH;
         sr->in_base = 0;
-        fill_side(&sr->p.in, &im->lay_s[sr->in_lay], nd, 0);
+        li = &im->lay_s[sr->in_lay];
+        fill_side(&sr->p.in, li, nd, 0);
       }
       if (sr->out_buf == BUF_WORK && sr->out_base != 0) {
         sr->out_buf = BUF_SCRATCH;
         sr->out_base = 0;
-        fill_side(&sr->p.out, &im->lay_s[sr->out_lay], nd, 0);
+        lo = &im->lay_s[sr->out_lay];
+        fill_side(&sr->p.out, lo, nd, 0);
       }
+      sr->p.reg = reg_form(im, &sr->p, li, lo);
     }
   }
   /* a plan small enough for dmg_split_run_noalloc: make the module that
@@ -663,6 +700,9 @@ static int impl_upload(struct dmg_split_impl *im) {
 static const char *side_kind(int sep, int semi, int pair) {
   return pair ? "(paired)" : sep ? "" : (semi ? "(shared dim)" : "(per value)");
 }
+
+/* lines in registers, and the axis along which lanes run */
+static const char *const reg_name[3] = {"", " regs=v1", " regs=t"};
 
 /* A pass's tile axes fastest first in memory, as letters: t the transform
  * axis, a and b the first and second vector axes. */
@@ -712,6 +752,7 @@ static int build_passes_split(struct dmg_split_impl *im) {
      * after its transform; the factor is constant along the other dimensions'
      * lines, so it commutes with the remaining stage-1 passes */
     f->p.twiddle = (stage[k] == 1 && K > n1 && im->A[subs[k] / 2] > 1) ? 1 : 0;
+    f->p.reg = reg_form(im, &f->p, &im->lay[in_lay], &im->lay[out_lay]);
   }
   for (int k = 0; k < K; ++k) {
     /* inverse pass k undoes forward pass K-1-k: it reads what that pass
@@ -730,20 +771,21 @@ static int build_passes_split(struct dmg_split_impl *im) {
     b->line = 0;
     b->p.sign = +1;
     b->p.twiddle = f->p.twiddle ? 2 : 0;
+    b->p.reg = reg_form(im, &b->p, &im->lay[b->in_lay], &im->lay[b->out_lay]);
   }
   im->lines = 0;
   int pos = snprintf(im->desc, sizeof(im->desc), "A=[%d,%d,%d] B=[%d,%d,%d] split passes=%d:", im->A[0],
                      nd > 1 ? im->A[1] : 1, nd > 2 ? im->A[2] : 1, im->B[0], nd > 1 ? im->B[1] : 1,
                      nd > 2 ? im->B[2] : 1, K);
-  for (int k = 0; k < K && pos < (int)sizeof(im->desc) - 64; ++k) {
+  for (int k = 0; k < K && pos < (int)sizeof(im->desc) - 112; ++k) {
     const struct dmg_fft_pass *p = &im->fwd[k].p;
     char lo[4], so[4];
     axis_letters(p->load_order, lo);
     axis_letters(p->store_order, so);
     pos += snprintf(im->desc + pos, sizeof(im->desc) - pos,
-                    " [t=%d n=%d v1=%d x%d v2=%d x%d tiles=%lld%s in=%s%s out=%s%s]", p->t, p->n, p->v1, p->M1, p->v2,
+                    " [t=%d n=%d v1=%d x%d v2=%d x%d tiles=%lld%s in=%s%s out=%s%s%s]", p->t, p->n, p->v1, p->M1, p->v2,
                     p->M2, (long long)p->ntiles, p->twiddle ? " tw" : "", lo, side_kind(p->sep_in, p->semi_in, p->pair_in), so,
-                    side_kind(p->sep_out, p->semi_out, p->pair_out));
+                    side_kind(p->sep_out, p->semi_out, p->pair_out), reg_name[p->reg]);
   }
   return DMG_OK;
 }
@@ -792,6 +834,7 @@ static int build_passes_line(struct dmg_split_impl *im) {
       f->p.perm_a = im->A[d];
       f->p.perm_b = im->B[d];
     }
+    f->p.reg = reg_form(im, &f->p, &im->lay[f->in_lay], &im->lay[f->out_lay]);
   }
   for (int k = 0; k < K; ++k) {
     const pass_rec *f = &im->fwd[K - 1 - k];
@@ -809,21 +852,22 @@ static int build_passes_line(struct dmg_split_impl *im) {
     b->p.perm_in = f->p.perm_out;
     b->p.perm_a = f->p.perm_a;
     b->p.perm_b = f->p.perm_b;
+    b->p.reg = reg_form(im, &b->p, &im->lay[b->in_lay], &im->lay[b->out_lay]);
   }
   im->lines = 1;
   int pos = snprintf(im->desc, sizeof(im->desc), "A=[%d,%d,%d] B=[%d,%d,%d] lines passes=%d:", im->A[0],
                      nd > 1 ? im->A[1] : 1, nd > 2 ? im->A[2] : 1, im->B[0], nd > 1 ? im->B[1] : 1,
                      nd > 2 ? im->B[2] : 1, K);
-  for (int k = 0; k < K && pos < (int)sizeof(im->desc) - 64; ++k) {
+  for (int k = 0; k < K && pos < (int)sizeof(im->desc) - 112; ++k) {
     const struct dmg_fft_pass *p = &im->fwd[k].p;
     char lo[4], so[4];
     axis_letters(p->load_order, lo);
     axis_letters(p->store_order, so);
     pos += snprintf(im->desc + pos, sizeof(im->desc) - pos,
-                    " [d=%d n=%d v1=%d x%d v2=%d x%d tiles=%lld%s in=%s%s out=%s%s]", p->t / 2, p->n,
+                    " [d=%d n=%d v1=%d x%d v2=%d x%d tiles=%lld%s in=%s%s out=%s%s%s]", p->t / 2, p->n,
                     p->v1 >= 0 ? p->v1 / 2 : -1, p->M1, p->v2 >= 0 ? p->v2 / 2 : -1, p->M2, (long long)p->ntiles,
                     p->perm_out ? " slots" : "", lo, side_kind(p->sep_in, p->semi_in, p->pair_in), so,
-                    side_kind(p->sep_out, p->semi_out, p->pair_out));
+                    side_kind(p->sep_out, p->semi_out, p->pair_out), reg_name[p->reg]);
   }
   return DMG_OK;
 }

@@ -20,7 +20,37 @@ int dmg_fft_pass_f32_inv_group(const dmg_fft_group *g, void *stream);
 int dmg_fft_pass_df_fwd_group(const dmg_fft_group *g, void *stream);
 int dmg_fft_pass_df_inv_group(const dmg_fft_group *g, void *stream);
 
+// passes with their lines in registers (fft_reg_*.cu)
+#define DMG_REG_DECL(a)                                                                    \
+  int dmg_fft_reg_##a##_fwd_v(const dmg_fft_pass *p, const dmg_fft_batch *b, void *stream); \
+  int dmg_fft_reg_##a##_fwd_t(const dmg_fft_pass *p, const dmg_fft_batch *b, void *stream); \
+  int dmg_fft_reg_##a##_inv_v(const dmg_fft_pass *p, const dmg_fft_batch *b, void *stream); \
+  int dmg_fft_reg_##a##_inv_t(const dmg_fft_pass *p, const dmg_fft_batch *b, void *stream);
+DMG_REG_DECL(f64)
+DMG_REG_DECL(f32)
+DMG_REG_DECL(df)
+#undef DMG_REG_DECL
+
 namespace {
+
+// A pass's lines over every job, as the register kernels number them.
+int64_t reg_line_count(const dmg_fft_pass &p, const dmg_fft_batch &b) {
+  int64_t n = (int64_t)b.count * p.nv1 * p.nv2;
+  for (int i = 0; i < p.nbatch; ++i) n *= p.blen[i];
+  return n;
+}
+
+int launch_reg(const dmg_fft_pass *p, int dtype, const dmg_fft_batch *b, void *stream) {
+  const int st = dtype == 0 ? check_batch<double>(*p, *b) : dtype == 2 ? check_batch<df>(*p, *b) : check_batch<float>(*p, *b);
+  if (st != DMG_OK) return st;
+  const bool t = p->reg == DMG_FFT_REG_T, inv = p->sign > 0;
+  using launcher = int (*)(const dmg_fft_pass *, const dmg_fft_batch *, void *);
+  static const launcher table[3][2][2] = {
+      {{dmg_fft_reg_f64_fwd_v, dmg_fft_reg_f64_fwd_t}, {dmg_fft_reg_f64_inv_v, dmg_fft_reg_f64_inv_t}},
+      {{dmg_fft_reg_f32_fwd_v, dmg_fft_reg_f32_fwd_t}, {dmg_fft_reg_f32_inv_v, dmg_fft_reg_f32_inv_t}},
+      {{dmg_fft_reg_df_fwd_v, dmg_fft_reg_df_fwd_t}, {dmg_fft_reg_df_inv_v, dmg_fft_reg_df_inv_t}}};
+  return table[dtype == 3 ? 1 : dtype][inv][t](p, b, stream);
+}
 
 // Largest biased exponent of max(|re|, |im|) over every element of a layout.
 // Coordinates enumerate the global array in C order; dimensions beyond ndim
@@ -85,6 +115,8 @@ extern "C" int dmg_fft_pass_launch_batch(const dmg_fft_pass *p, int dtype, const
     return dmg_error(DMG_ERR_ARG, "fft pass: wide tiles for length %d in arithmetic %d", p->n, dtype);
   if ((p->perm_in || p->perm_out) && (p->perm_a < 1 || p->perm_b < 1 || (int64_t)p->perm_a * p->perm_b != p->n))
     return dmg_error(DMG_ERR_ARG, "fft slot order %d x %d does not match length %d", p->perm_a, p->perm_b, p->n);
+  // (the register kernels number lines in 31 bits)
+  if (p->reg && dtype >= 0 && dtype <= 3 && reg_line_count(*p, *b) < ((int64_t)1 << 31)) return launch_reg(p, dtype, b, stream);
   switch (dtype) {
     case 0: return dmg_fft_pass_launch_f64(p, b, stream);
     case 1: return dmg_fft_pass_launch_f32(p, b, stream);

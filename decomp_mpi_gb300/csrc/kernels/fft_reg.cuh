@@ -1,0 +1,978 @@
+// FFT passes whose lines live in registers: the kernel of every pass whose
+// length has a schedule here, whose sides are separable and whose sides run
+// along the same fastest tile axis (fft_pass.cuh serves the rest).
+//
+// A block transforms W whole lines at a time with TL threads per line.  A
+// thread loads the R values of its first butterfly straight from the input
+// layout into registers, transforms them, and exchanges them with the line's
+// other threads through shared memory once per further stage (n = R1 R2: one
+// exchange, R1 R2 R3: two); the last stage's results go from registers to the
+// output layout.  What bounds the kernels of fft_pass.cuh is not HBM but
+// their instruction count (FP32 100 instructions per value, half of them
+// index arithmetic; double-float 296; native FP64 219) at 16 warps per SM.
+// Here a value costs one table read, one 64-bit address addition and one
+// access per side; every shared-memory position is a thread's base plus a
+// compile-time constant, and a line's values cross shared memory once or
+// twice instead of four times.
+//
+// Lines.  A pass's lines (all tile and batch axes and the jobs of a batch)
+// are numbered along v1, then v2, then the batch axes, then the jobs, and a
+// block takes W consecutive ones, so that extents that do not divide by a
+// tile leave no lanes idle except in the last tile.  A line's address on a
+// side is the sum of its dimensions' table entries; the transform axis adds
+// an offset that is the same for every line (the host checks this), kept in
+// shared memory as int32 with the slot order of line passes folded in.
+//
+// Two forms: "along v1" (v1 is the fastest axis on both sides: neighbouring
+// lanes hold neighbouring lines, shared memory is [position][line]) and
+// "along t" (the transform axis is: neighbouring lanes hold neighbouring
+// values of a line, shared memory is [line][position]).  Along t, a side in
+// slot order is read or written in that order through one more exchange, so
+// that its accesses stay contiguous.
+//
+// Measured on one GB300 against the tiled kernel (forward transforms, lines
+// schedule): 1024^3 complex64 FP32 26.1 -> 12.1 ms (a pass's bytes at the
+// copy rate: 2.53 ms); 8 cubes of 240^3 complex64, forward and back, 6.43 ->
+// 2.59 ms; 512^3 complex128 double-float 7.95 -> 5.78 ms, native FP64 step
+// (forward, inverse and two reshapes) 38.6 -> 37.7 ms, where the FP64 pipe
+// binds.
+#pragma once
+#include "fft_pass.cuh"
+
+namespace {
+
+// ---------------------------------------------------------------- schedules
+
+// Radices, threads per line, lines per block and resident blocks per SM the
+// register budget allows.  kind: 0 native FP64, 1 FP32, 2 double-float.
+struct RegSched {
+  int ns;
+  int r[3];
+  int tl, w, minb;
+};
+
+__host__ __device__ constexpr RegSched reg_sched(int kind, int n) {
+  if (kind == 1) {
+    switch (n) {
+      case 32: return {2, {8, 4, 1}, 4, 64, 3};
+      case 48: return {2, {8, 6, 1}, 8, 32, 3};
+      case 64: return {2, {8, 8, 1}, 8, 32, 3};
+      case 96: return {2, {12, 8, 1}, 12, 16, 3};
+      case 120: return {2, {12, 10, 1}, 12, 16, 3};
+      case 128: return {2, {16, 8, 1}, 8, 32, 3};
+      case 160: return {2, {16, 10, 1}, 16, 16, 3};
+      case 192: return {2, {16, 12, 1}, 16, 16, 3};
+      case 240: return {2, {16, 15, 1}, 16, 16, 3};
+      case 256: return {2, {16, 16, 1}, 16, 16, 3};
+      case 320: return {2, {20, 16, 1}, 20, 8, 3};
+      case 384: return {2, {24, 16, 1}, 24, 8, 3};
+      case 480: return {2, {24, 20, 1}, 24, 8, 3};
+      case 512: return {2, {32, 16, 1}, 16, 16, 2};
+      case 1024: return {2, {32, 32, 1}, 32, 8, 2};
+      case 2048: return {3, {16, 16, 8}, 128, 4, 2};
+      default: return {0, {1, 1, 1}, 1, 1, 1};
+    }
+  }
+  if (kind == 0) {
+    switch (n) {
+      case 32: return {2, {8, 4, 1}, 4, 32, 3};
+      case 48: return {2, {8, 6, 1}, 8, 16, 4};
+      case 64: return {2, {8, 8, 1}, 8, 16, 4};
+      case 96: return {2, {12, 8, 1}, 12, 8, 4};
+      case 120: return {2, {12, 10, 1}, 12, 8, 4};
+      case 128: return {2, {16, 8, 1}, 8, 16, 3};
+      case 160: return {2, {16, 10, 1}, 16, 8, 3};
+      case 192: return {2, {16, 12, 1}, 16, 8, 3};
+      case 240: return {2, {16, 15, 1}, 16, 8, 3};
+      case 256: return {2, {16, 16, 1}, 16, 8, 3};
+      case 320: return {3, {8, 10, 4}, 40, 4, 3};
+      case 384: return {3, {8, 12, 4}, 48, 4, 2};
+      case 480: return {3, {12, 10, 4}, 48, 4, 2};
+      case 512: return {3, {8, 8, 8}, 64, 4, 2};
+      case 1024: return {3, {8, 16, 8}, 64, 4, 2};
+      default: return {0, {1, 1, 1}, 1, 1, 1};
+    }
+  }
+  switch (n) {
+    case 32: return {2, {8, 4, 1}, 4, 32, 3};
+    case 48: return {2, {8, 6, 1}, 8, 32, 2};
+    case 64: return {2, {8, 8, 1}, 8, 32, 2};
+    case 96: return {2, {12, 8, 1}, 12, 16, 2};
+    case 120: return {2, {12, 10, 1}, 12, 16, 2};
+    case 128: return {3, {8, 4, 4}, 16, 16, 2};
+    case 160: return {3, {8, 5, 4}, 20, 8, 3};
+    case 192: return {3, {8, 6, 4}, 24, 8, 2};
+    case 240: return {3, {8, 6, 5}, 30, 8, 2};
+    case 256: return {3, {8, 8, 4}, 32, 8, 2};
+    case 320: return {3, {8, 10, 4}, 40, 4, 3};
+    case 384: return {3, {8, 12, 4}, 48, 4, 2};
+    case 480: return {3, {12, 10, 4}, 48, 4, 2};
+    case 512: return {3, {8, 8, 8}, 64, 4, 2};
+    case 1024: return {3, {8, 16, 8}, 64, 4, 2};
+    default: return {0, {1, 1, 1}, 1, 1, 1};
+  }
+}
+template <typename T>
+__host__ __device__ constexpr int reg_kind() {
+  return std::is_same<T, float>::value ? 1 : std::is_same<T, df>::value ? 2 : 0;
+}
+__host__ __device__ constexpr bool is_pow2(int n) { return n > 0 && (n & (n - 1)) == 0; }
+
+// ---------------------------------------------------------------- butterflies in registers
+
+// a * b with scalar FMAs in FP32 (the paired form has to build pairs of equal values first)
+template <typename T>
+__device__ __forceinline__ C2<T> rmul(C2<T> a, C2<T> b) {
+  if constexpr (std::is_same<T, float>::value) {
+    return make_float2(fmaf(a.x, b.x, -(a.y * b.y)), fmaf(a.x, b.y, a.y * b.x));
+  } else {
+    return mul<T>(a, b);
+  }
+}
+// a + sign i b and a - sign i b
+template <typename T, int SIGN, bool LAZY = false>
+__device__ __forceinline__ C2<T> add_rot(C2<T> a, C2<T> b) {
+  if constexpr (std::is_same<T, df>::value) {
+    return LAZY ? addl<T>(a, rot90<T, SIGN>(b)) : add<T>(a, rot90<T, SIGN>(b));
+  } else {
+    C2<T> r;
+    r.x = SIGN < 0 ? a.x + b.y : a.x - b.y;
+    r.y = SIGN < 0 ? a.y - b.x : a.y + b.x;
+    return r;
+  }
+}
+template <typename T, int SIGN, bool LAZY = false>
+__device__ __forceinline__ C2<T> sub_rot(C2<T> a, C2<T> b) {
+  return add_rot<T, -SIGN, LAZY>(a, b);
+}
+
+// cos(pi k / 16), k = 0 ... 8, as a double and as two floats
+template <typename T, int K>
+__device__ __forceinline__ T cos16() {
+  static_assert(K >= 0 && K <= 8, "first quadrant");
+  if constexpr (K == 0) return cst<T>(1.0, 1.0f, 0.0f);
+  else if constexpr (K == 1) return cst<T>(0.980785280403230449126182236134239036, 0.9807852506637573f, 2.9739473106360492e-08f);
+  else if constexpr (K == 2) return cst<T>(0.923879532511286756128183189396788286, 0.9238795042037964f, 2.830748968563057e-08f);
+  else if constexpr (K == 3) return cst<T>(0.831469612302545237078788377617905756, 0.8314695954322815f, 1.687026340846387e-08f);
+  else if constexpr (K == 4) return cst<T>(K_SQRT1_2);
+  else if constexpr (K == 5) return cst<T>(0.555570233019602224742830813948532874, 0.5555702447891235f, -1.1769521357507529e-08f);
+  else if constexpr (K == 6) return cst<T>(0.382683432365089771728459984030398866, 0.3826834261417389f, 6.2233507236442165e-09f);
+  else if constexpr (K == 7) return cst<T>(0.195090322016128267848284868477022240, 0.19509032368659973f, -1.670471427850373e-09f);
+  else return cst<T>(0.0, 0.0f, 0.0f);
+}
+template <typename T>
+__device__ __forceinline__ T rneg(T a) { return -a; }
+// exp(sign i pi K / 16) as (re, im), any K
+template <typename T, int SIGN, int K>
+__device__ __forceinline__ void unit16(T &re, T &im) {
+  constexpr int k = ((K % 32) + 32) % 32;
+  constexpr int q = k / 8, r = k % 8;  // quadrant, angle within it
+  const T c = cos16<T, r>(), s = cos16<T, 8 - r>();
+  // e^{i (q pi/2 + a)} = i^q (c + i s)
+  T x = q == 0 ? c : q == 1 ? rneg(s) : q == 2 ? rneg(c) : s;
+  T y = q == 0 ? s : q == 1 ? c : q == 2 ? rneg(s) : rneg(c);
+  re = x;
+  im = SIGN < 0 ? rneg(y) : y;
+}
+__device__ __forceinline__ float2 pack_c(float x, float y) { return make_float2(x, y); }
+__device__ __forceinline__ double2 pack_c(double x, double y) { return make_double2(x, y); }
+__device__ __forceinline__ dfc pack_c(df x, df y) { return dfc{make_float2(x.h, y.h), make_float2(x.l, y.l)}; }
+// v * exp(sign 2 pi i E / R), R a power of two up to 32
+template <typename T, int SIGN, int R, int E>
+__device__ __forceinline__ C2<T> mul_unit(C2<T> v) {
+  constexpr int K = (E * (32 / R)) % 32;
+  if constexpr (K == 0) {
+    return v;
+  } else if constexpr (K == 8) {
+    return rot90<T, SIGN>(v);
+  } else if constexpr (K % 8 == 4) {
+    // (+-1 +- i) / sqrt 2: a sum with the rotated value, scaled
+    const T c = cst<T>(K_SQRT1_2);
+    if constexpr (K == 4) return scl<T>(add_rot<T, SIGN, true>(v, v), c);
+    else return scl<T>(subl<T>(rot90<T, SIGN>(v), v), c);  // K == 12
+  } else if constexpr (std::is_same<T, float>::value) {
+    // The FP32 roundings of these few constants all make the factor shorter (by up to 2.9e-8): the trailing
+    // part of the longer component goes in too, which keeps the bias from adding up over stages and passes
+    // (1024-point round trip 2.39e-7 without it, 2.18e-7 in the tiled kernel's radix-8 and -4 stages).
+    df re, im;
+    unit16<df, SIGN, K>(re, im);
+    constexpr int k = K % 16;
+    if constexpr (k < 4 || k > 12) {
+      return make_float2(fmaf(v.x, re.h, fmaf(v.x, re.l, -(v.y * im.h))), fmaf(v.y, re.h, fmaf(v.y, re.l, v.x * im.h)));
+    } else {
+      return make_float2(fmaf(-v.y, im.h, fmaf(-v.y, im.l, v.x * re.h)), fmaf(v.x, im.h, fmaf(v.x, im.l, v.y * re.h)));
+    }
+  } else {
+    T re, im;
+    unit16<T, SIGN, K>(re, im);
+    return rmul<T>(v, pack_c(re, im));
+  }
+}
+
+template <typename T, int SIGN, bool LAZY = false>
+__device__ __forceinline__ void rdft4(C2<T> &a0, C2<T> &a1, C2<T> &a2, C2<T> &a3) {
+  const C2<T> t0 = addl<T>(a0, a2), t1 = subl<T>(a0, a2), t2 = addl<T>(a1, a3), t3 = subl<T>(a1, a3);
+  if constexpr (LAZY) {
+    a0 = addl<T>(t0, t2);
+    a2 = subl<T>(t0, t2);
+  } else {
+    a0 = add<T>(t0, t2);
+    a2 = sub<T>(t0, t2);
+  }
+  a1 = add_rot<T, SIGN, LAZY>(t1, t3);
+  a3 = sub_rot<T, SIGN, LAZY>(t1, t3);
+}
+template <typename T, int SIGN>
+__device__ __forceinline__ void rdft8(C2<T> *a) {
+  if constexpr (std::is_same<T, float>::value) {
+    C2<T> e0 = a[0], e1 = a[2], e2 = a[4], e3 = a[6];
+    C2<T> o0 = a[1], o1 = a[3], o2 = a[5], o3 = a[7];
+    rdft4<T, SIGN>(e0, e1, e2, e3);
+    rdft4<T, SIGN>(o0, o1, o2, o3);
+    // o1 (1 + sign i) / sqrt 2 and o3 (-1 + sign i) / sqrt 2, the scale inside the last additions
+    const float c = 0.70710678118654752440f;
+    const float2 w1 = add_rot<T, SIGN>(o1, o1);
+    const float2 w3 = make_float2(SIGN < 0 ? o3.y - o3.x : -o3.y - o3.x, SIGN < 0 ? -o3.x - o3.y : o3.x - o3.y);
+    a[0] = cadd(e0, o0);
+    a[4] = csub(e0, o0);
+    a[1] = pfma(w1, splat(c), e1);
+    a[5] = pfma(w1, splat(-c), e1);
+    a[2] = add_rot<T, SIGN>(e2, o2);
+    a[6] = sub_rot<T, SIGN>(e2, o2);
+    a[3] = pfma(w3, splat(c), e3);
+    a[7] = pfma(w3, splat(-c), e3);
+  } else {
+    dft8<T, SIGN>(a);
+  }
+}
+template <typename T, int SIGN>
+__device__ __forceinline__ void rdft3(C2<T> *a) {
+  const C2<T> s = add<T>(a[1], a[2]);
+  const C2<T> d = sub<T>(a[1], a[2]);
+  const C2<T> m = sub<T>(a[0], scl<T>(s, cst<T>(K_HALF)));
+  const C2<T> r = scl<T>(d, cst<T>(K_SQRT3_2));
+  a[0] = add<T>(a[0], s);
+  a[1] = add_rot<T, SIGN>(m, r);
+  a[2] = sub_rot<T, SIGN>(m, r);
+}
+template <typename T, int SIGN>
+__device__ __forceinline__ void rdft5(C2<T> *a) {
+  const C2<T> b1 = add<T>(a[1], a[4]), b2 = add<T>(a[2], a[3]);
+  const C2<T> d1 = sub<T>(a[1], a[4]), d2 = sub<T>(a[2], a[3]);
+  const T c1 = cst<T>(K_C72), c2 = cst<T>(K_C144), s1 = cst<T>(K_S72), s2 = cst<T>(K_S144);
+  const C2<T> p1 = add<T>(a[0], add<T>(scl<T>(b1, c1), scl<T>(b2, c2)));
+  const C2<T> p2_ = add<T>(a[0], add<T>(scl<T>(b1, c2), scl<T>(b2, c1)));
+  const C2<T> q1 = add<T>(scl<T>(d1, s1), scl<T>(d2, s2));
+  const C2<T> q2 = sub<T>(scl<T>(d1, s2), scl<T>(d2, s1));
+  a[0] = add<T>(a[0], add<T>(b1, b2));
+  a[1] = add_rot<T, SIGN>(p1, q1);
+  a[4] = sub_rot<T, SIGN>(p1, q1);
+  a[2] = add_rot<T, SIGN>(p2_, q2);
+  a[3] = sub_rot<T, SIGN>(p2_, q2);
+}
+
+template <typename T, int SIGN, int R>
+__device__ __forceinline__ void rdft(C2<T> *a);
+
+// twiddles of the inner products: column k1 of row i2 times exp(sign 2 pi i i2 k1 / R)
+template <typename T, int SIGN, int R, int A, int B, int I2, int K1>
+__device__ __forceinline__ void ct_twiddle(C2<T> *row) {
+  if constexpr (K1 < A) {
+    row[K1] = mul_unit<T, SIGN, R, I2 * K1>(row[K1]);
+    ct_twiddle<T, SIGN, R, A, B, I2, K1 + 1>(row);
+  }
+}
+template <typename T, int SIGN, int R, int A, int B, int I2>
+__device__ __forceinline__ void ct_rows(C2<T> (*y)[A], const C2<T> *a) {
+  if constexpr (I2 < B) {
+#pragma unroll
+    for (int i1 = 0; i1 < A; ++i1) y[I2][i1] = a[i1 * B + I2];
+    rdft<T, SIGN, A>(y[I2]);
+    ct_twiddle<T, SIGN, R, A, B, I2, 1>(y[I2]);
+    ct_rows<T, SIGN, R, A, B, I2 + 1>(y, a);
+  }
+}
+// R = A B, powers of two: DFTs of A over the stride-B columns, twiddles, DFTs of B
+template <typename T, int SIGN, int R, int A>
+__device__ __forceinline__ void dft_ct(C2<T> *a) {
+  constexpr int B = R / A;
+  C2<T> y[B][A];
+  ct_rows<T, SIGN, R, A, B, 0>(y, a);
+#pragma unroll
+  for (int k1 = 0; k1 < A; ++k1) {
+    C2<T> z[B];
+#pragma unroll
+    for (int i2 = 0; i2 < B; ++i2) z[i2] = y[i2][k1];
+    rdft<T, SIGN, B>(z);
+#pragma unroll
+    for (int k2 = 0; k2 < B; ++k2) a[k1 + A * k2] = z[k2];
+  }
+}
+// the x of [0, m) with a x = 1 mod m
+__host__ __device__ constexpr int mod_inverse(int a, int m) {
+  for (int x = 1; x < m; ++x)
+    if (a * x % m == 1) return x;
+  return 0;
+}
+// R = A B, coprime: no twiddles (Good's index maps: input B i1 + A i2, output the k with remainders k1 mod A
+// and k2 mod B)
+template <typename T, int SIGN, int R, int A>
+__device__ __forceinline__ void dft_pfa(C2<T> *a) {
+  constexpr int B = R / A;
+  constexpr int EA = B * mod_inverse(B, A), EB = A * mod_inverse(A, B);
+  C2<T> y[B][A];
+#pragma unroll
+  for (int i2 = 0; i2 < B; ++i2) {
+#pragma unroll
+    for (int i1 = 0; i1 < A; ++i1) y[i2][i1] = a[(B * i1 + A * i2) % R];
+    rdft<T, SIGN, A>(y[i2]);
+  }
+#pragma unroll
+  for (int k1 = 0; k1 < A; ++k1) {
+    C2<T> z[B];
+#pragma unroll
+    for (int i2 = 0; i2 < B; ++i2) z[i2] = y[i2][k1];
+    rdft<T, SIGN, B>(z);
+#pragma unroll
+    for (int k2 = 0; k2 < B; ++k2) {
+      a[(EA * k1 + EB * k2) % R] = z[k2];
+    }
+  }
+}
+
+template <typename T, int SIGN, int R>
+__device__ __forceinline__ void rdft(C2<T> *a) {
+  if constexpr (R == 1) {
+  } else if constexpr (R == 2) {
+    const C2<T> t = add<T>(a[0], a[1]);
+    a[1] = sub<T>(a[0], a[1]);
+    a[0] = t;
+  } else if constexpr (R == 3) {
+    rdft3<T, SIGN>(a);
+  } else if constexpr (R == 4) {
+    rdft4<T, SIGN>(a[0], a[1], a[2], a[3]);
+  } else if constexpr (R == 5) {
+    rdft5<T, SIGN>(a);
+  } else if constexpr (R == 8) {
+    rdft8<T, SIGN>(a);
+  } else if constexpr (R == 16) {
+    dft_ct<T, SIGN, 16, 4>(a);
+  } else if constexpr (R == 32) {
+    dft_ct<T, SIGN, 32, 4>(a);
+  } else if constexpr (R % 8 == 0) {
+    dft_pfa<T, SIGN, R, 8>(a);  // 24
+  } else if constexpr (R % 4 == 0) {
+    dft_pfa<T, SIGN, R, 4>(a);  // 12, 20
+  } else if constexpr (R % 2 == 0) {
+    dft_pfa<T, SIGN, R, 2>(a);  // 6, 10
+  } else {
+    static_assert(R == 15, "radix");
+    dft_pfa<T, SIGN, R, 3>(a);
+  }
+}
+
+// Native FP64, power-of-two radix R: every layer as radix-2 butterflies
+// y0 = a + t b, y1 = 2 a - y0 (six FMAs; four additions where t is a quarter
+// turn), the stage's input twiddles w^q included.  With n values x_q whose
+// factors are u^q (u = w W_R^e), the even outputs are the n/2 values
+// x_q + u^{n/2} x_{q+n/2} with factors u^q, the odd ones their differences
+// with factors (u W_n)^q; level d so needs w^{R / 2^{d+1}} W_{2^{d+1}}^e for
+// e < 2^d, the upper half of them a quarter turn from the lower.  tw: those
+// entries, [w^{R/2}], [w^{R/4}], [w^{R/8}, w^{R/8} W_8], ...  Outputs in
+// bit-reversed places.
+__host__ __device__ constexpr int fma_entries(int R) { return R <= 2 ? R - 1 : R / 2; }
+__host__ __device__ constexpr int bit_reverse(int k, int R) {
+  int r = 0;
+  for (int b = 1; b < R; b <<= 1) {
+    r = (r << 1) | (k & 1);
+    k >>= 1;
+  }
+  return r;
+}
+// level d, e in the lower half (e < 2^{d-1}, or d = 0)
+__host__ __device__ constexpr int fma_entry(int d, int e) { return d == 0 ? 0 : (1 << (d - 1)) + e; }
+
+template <int SIGN>
+__device__ __forceinline__ void bfly_plain(double2 &a, double2 &b) {
+  const double2 t = cadd(a, b);
+  b = csub(a, b);
+  a = t;
+}
+template <int SIGN>
+__device__ __forceinline__ void bfly_plain_rot(double2 &a, double2 &b) {
+  const double2 t = add_rot<double, SIGN>(a, b);
+  b = sub_rot<double, SIGN>(a, b);
+  a = t;
+}
+// TW: with input twiddles (else w = 1); N values at a, level D, twiddle exponent E
+template <int SIGN, int R, bool TW, int N, int D, int E>
+__device__ __forceinline__ void fma_node(double2 *a, const double2 *tw) {
+  if constexpr (N > 1) {
+    constexpr int H = N / 2;
+    constexpr int HALF = D > 0 ? 1 << (D - 1) : 1;  // e and e + HALF differ by a quarter turn
+    constexpr int EL = D > 0 ? E % HALF : 0;
+    constexpr bool ROT = D > 0 && E >= HALF;
+    if constexpr (TW) {
+      const double2 t = tw[fma_entry(D, EL)];
+#pragma unroll
+      for (int q = 0; q < H; ++q) {
+        if constexpr (ROT) bfly_tw_rot<SIGN>(a[q], a[q + H], t.x, t.y);
+        else bfly_tw<SIGN>(a[q], a[q + H], t.x, t.y);
+      }
+    } else if constexpr (EL == 0) {
+#pragma unroll
+      for (int q = 0; q < H; ++q) {
+        if constexpr (ROT) bfly_plain_rot<SIGN>(a[q], a[q + H]);
+        else bfly_plain<SIGN>(a[q], a[q + H]);
+      }
+    } else if constexpr (E * (32 >> (D + 1)) % 8 == 4) {
+      // an odd eighth turn: (1 + sign i) b or (-1 + sign i) b by additions, its scale in the outputs' FMAs
+      // (six operations as well, without the difference's doubled rounding)
+      const double c = 0.707106781186547524400844362104849039;
+#pragma unroll
+      for (int q = 0; q < H; ++q) {
+        const double2 b = a[q + H];
+        double2 w = add_rot<double, SIGN>(b, b);
+        if constexpr (ROT) w = SIGN < 0 ? make_double2(w.y, -w.x) : make_double2(-w.y, w.x);
+        a[q + H] = make_double2(__fma_rn(-c, w.x, a[q].x), __fma_rn(-c, w.y, a[q].y));
+        a[q] = make_double2(__fma_rn(c, w.x, a[q].x), __fma_rn(c, w.y, a[q].y));
+      }
+    } else {
+      double re, im;
+      unit16<double, SIGN, E * (32 >> (D + 1))>(re, im);
+#pragma unroll
+      for (int q = 0; q < H; ++q) bfly_tw<SIGN>(a[q], a[q + H], re, im);
+    }
+    fma_node<SIGN, R, TW, H, D + 1, E>(a, tw);
+    fma_node<SIGN, R, TW, H, D + 1, E + (1 << D)>(a + H, tw);
+  }
+}
+
+// ---------------------------------------------------------------- the lines of a pass
+
+// An axis the lines are numbered along: its length (with the constants of a
+// division by it), its dimension, the coordinate step and whether it is the
+// twiddle's y.
+struct reg_axis {
+  uint32_t len, magic, shift;
+  int32_t dim, mul, isy;
+};
+struct reg_lines {
+  uint32_t total;  // lines of all jobs
+  uint32_t nax;
+  reg_axis ax[5];
+};
+// r / len for r < 2^31
+__device__ __forceinline__ uint32_t fast_div(uint32_t r, const reg_axis &a) {
+  return (__umulhi(r, a.magic) + r) >> a.shift;
+}
+
+template <typename T, int NF>
+struct RegShape {
+  static constexpr RegSched S = reg_sched(reg_kind<T>(), NF);
+  static constexpr int TL = S.tl, W = S.w, NTH = TL * W;
+  static constexpr int ES = (int)sizeof(C2<T>);
+  static constexpr int V = 128 / ES;  // values per shared-memory wavefront
+  // stage f: radix, product of the earlier radices, values per row after it, butterflies, rounds per thread
+  static constexpr int R(int f) { return S.r[f]; }
+  static constexpr int LP(int f) { return f == 0 ? 1 : LP(f - 1) * S.r[f - 1]; }
+  static constexpr int M(int f) { return NF / (LP(f) * S.r[f]); }
+  static constexpr int NB(int f) { return NF / S.r[f]; }
+  static constexpr int TR(int f) { return (NB(f) + TL - 1) / TL; }
+  // The exchange after stage f holds row J (of LP R) and value k (of m) at
+  // J P + k; the next stage's thread (j', k') reads J = j', k = q m' + k'.
+  // The row pitch P leaves consecutive threads of the next stage in
+  // different banks: P an odd multiple of m' while m' is less than the lanes
+  // of a wavefront that run along the line (the lines take the others in the
+  // form along v1).
+  static constexpr int pitch(int f, bool tf) {
+    const int m = M(f), mn = M(f + 1);
+    const int lanes = !tf ? (W >= V ? 1 : V / W) : TL >= V ? V : TL >= 8 ? 8 : 4;
+    if (mn >= lanes || !is_pow2(mn)) return m;
+    int p = m;
+    while (p % (2 * mn) != mn) ++p;
+    return p;
+  }
+  static constexpr int rows(int f) { return LP(f) * S.r[f]; }
+  // slot-order exchange (along t): rows of M(0) values before the first stage, of LP(last) after the last
+  static constexpr int in_row = M(0), in_pitch = M(0) | 1;
+  static constexpr int out_row = LP(S.ns - 1), out_pitch = LP(S.ns - 1) | 1;
+  static constexpr int cmax(int a, int b) { return a > b ? a : b; }
+  static constexpr int line_values(bool tf) {
+    int v = 0;
+    for (int f = 0; f + 1 < S.ns; ++f) v = cmax(v, rows(f) * pitch(f, tf));
+    if (tf) v = cmax(v, cmax((NF / in_row) * in_pitch, (NF / out_row) * out_pitch));
+    return v;
+  }
+  // line pitch along t: the lines of a wavefront start in different banks
+  static constexpr int line_pitch() {
+    int v = line_values(true);
+    if (TL < V)
+      while (v % V != TL % V) ++v;
+    return v;
+  }
+  static constexpr size_t buf_bytes(bool tf) { return (size_t)W * (tf ? line_pitch() : line_values(false)) * ES; }
+  // twiddle table entries per j of stage f
+  static constexpr bool fma(int f) { return std::is_same<T, double>::value && is_pow2(S.r[f]) && S.r[f] <= 32; }
+  static constexpr int tw_per_j(int f) { return f == 0 ? 0 : fma(f) ? fma_entries(S.r[f]) : S.r[f] - 1; }
+  static constexpr int tw_base(int f) { return f <= 1 ? 0 : tw_base(f - 1) + tw_per_j(f - 1) * LP(f - 1); }
+  static constexpr int tw_total() { return tw_base(S.ns - 1) + tw_per_j(S.ns - 1) * LP(S.ns - 1); }
+  static constexpr size_t al16(size_t x) { return (x + 15) & ~(size_t)15; }
+  // shared memory: exchange buffer, twiddles, the sides' offsets (8 bytes a slot on the side that may be in
+  // slot order along t: the output forward, the input inverse), line pointers
+  static constexpr size_t tw_off(bool tf) { return al16(buf_bytes(tf)); }
+  static constexpr size_t tin_off(bool tf) { return al16(tw_off(tf) + (size_t)tw_total() * ES); }
+  static constexpr size_t tout_off(bool tf, int sign) { return al16(tin_off(tf) + (size_t)NF * (tf && sign > 0 ? 8 : 4)); }
+  static constexpr size_t ptr_off(bool tf, int sign) {
+    return al16(tout_off(tf, sign) + (size_t)NF * (tf && sign < 0 ? 8 : 4));
+  }
+  static constexpr size_t smem(bool tf, int sign) { return al16(ptr_off(tf, sign) + (tf ? (size_t)W * 8 : 0)); }
+};
+
+// ---------------------------------------------------------------- the kernel
+
+template <typename T, int SIGN, int NF, int F>
+__device__ __forceinline__ void reg_twiddles(const C2<T> *roots, C2<T> *tws, int tid) {
+  using G = RegShape<T, NF>;
+  if constexpr (F < G::S.ns) {
+    constexpr int LP = G::LP(F), R = G::R(F), PJ = G::tw_per_j(F), TS = NF / (LP * R);
+    for (int i = tid; i < PJ * LP; i += G::NTH) {
+      const int e = i / LP, j = i - e * LP;
+      int idx;
+      if constexpr (G::fma(F)) {
+        // level d, exponent e - 2^{d-1}: w^{R / 2^{d+1}} W_{2^{d+1}}^e
+        int d = 0;
+        while (d > 0 ? (e >> d) != 0 : e > 0) ++d;
+        const int x = d == 0 ? 0 : e - (1 << (d - 1));
+        idx = j * TS * (R >> (d + 1)) + x * (NF >> (d + 1));
+      } else {
+        idx = (e + 1) * j * TS;
+      }
+      tws[G::tw_base(F) + i] = root_at<T, SIGN>(roots, idx % NF);
+    }
+    reg_twiddles<T, SIGN, NF, F + 1>(roots, tws, tid);
+  }
+}
+
+// butterflies of stage F on the thread's registers, input twiddles included
+template <typename T, int SIGN, int NF, int F>
+__device__ __forceinline__ void reg_butterfly(C2<T> *a, const C2<T> *tws, int j) {
+  using G = RegShape<T, NF>;
+  constexpr int R = G::R(F), LP = G::LP(F);
+  const C2<T> *tw = tws + G::tw_base(F) + j;
+  if constexpr (G::fma(F)) {
+    if constexpr (F > 0) {
+      double2 t[fma_entries(R)];
+#pragma unroll
+      for (int e = 0; e < fma_entries(R); ++e) t[e] = tw[e * LP];
+      fma_node<SIGN, R, true, R, 0, 0>(a, t);
+    } else {
+      fma_node<SIGN, R, false, R, 0, 0>(a, nullptr);
+    }
+    C2<T> y[R];
+#pragma unroll
+    for (int s = 0; s < R; ++s) y[s] = a[bit_reverse(s, R)];
+#pragma unroll
+    for (int s = 0; s < R; ++s) a[s] = y[s];
+  } else {
+    if constexpr (F > 0) {
+#pragma unroll
+      for (int q = 1; q < R; ++q) a[q] = rmul<T>(a[q], tw[(q - 1) * LP]);
+    }
+    rdft<T, SIGN, R>(a);
+  }
+}
+
+// the stages from F on: the exchange into stage F's registers and its
+// butterflies; ends with the last stage's values in a (rounds of R each).
+// bx: the thread's first buffer position (its line's).  STEP: distance of
+// neighbouring positions of a line (W along v1, 1 along t).
+template <typename T, int SIGN, int NF, bool TF, int F>
+__device__ __forceinline__ void reg_exchange(const C2<T> *src, C2<T> *bx, const C2<T> *tws, int bl, C2<T> *out) {
+  using G = RegShape<T, NF>;
+  constexpr int STEP = TF ? 1 : G::W;
+  constexpr int P = G::pitch(F - 1, TF);
+  // write stage F - 1's results
+  {
+    constexpr int R = G::R(F - 1), LP = G::LP(F - 1), M = G::M(F - 1), NB = G::NB(F - 1), TR = G::TR(F - 1);
+    __syncthreads();  // the buffer's previous values have been read
+#pragma unroll
+    for (int tr = 0; tr < TR; ++tr) {
+      const int b = bl + tr * G::TL;
+      if (NB % G::TL == 0 || b < NB) {
+        C2<T> *w = bx + ((b / M) * P + b % M) * STEP;
+#pragma unroll
+        for (int s = 0; s < R; ++s) w[s * LP * P * STEP] = src[tr * R + s];
+      }
+    }
+    __syncthreads();
+  }
+  constexpr int R = G::R(F), M = G::M(F), NB = G::NB(F), TR = G::TR(F);
+  C2<T> a[TR * R];
+#pragma unroll
+  for (int tr = 0; tr < TR; ++tr) {
+    const int b = bl + tr * G::TL;
+    if (NB % G::TL == 0 || b < NB) {
+      const int j = b / M, k = b % M;
+      const C2<T> *x = bx + (j * P + k) * STEP;
+#pragma unroll
+      for (int q = 0; q < R; ++q) a[tr * R + q] = x[q * M * STEP];
+    }
+  }
+#pragma unroll
+  for (int tr = 0; tr < TR; ++tr) {
+    const int b = bl + tr * G::TL;
+    if (NB % G::TL == 0 || b < NB) reg_butterfly<T, SIGN, NF, F>(a + tr * R, tws, b / M);
+  }
+  if constexpr (F + 1 < G::S.ns) {
+    reg_exchange<T, SIGN, NF, TF, F + 1>(a, bx, tws, bl, out);
+  } else {
+#pragma unroll
+    for (int i = 0; i < TR * R; ++i) out[i] = a[i];
+  }
+}
+
+// a value as it lies in the input array (complex128 bits for a double-float pass that reads complex128)
+template <typename T>
+__device__ __forceinline__ C2<T> reg_load(const unsigned char *at) {
+  if constexpr (sizeof(C2<T>) == 16) {
+    const float4 v = *reinterpret_cast<const float4 *>(at);
+    C2<T> r;
+    memcpy(&r, &v, 16);
+    return r;
+  } else {
+    return *reinterpret_cast<const C2<T> *>(at);
+  }
+}
+template <typename T>
+__device__ __forceinline__ void reg_store(unsigned char *at, C2<T> v) {
+  if constexpr (sizeof(C2<T>) == 16) {
+    float4 w;
+    memcpy(&w, &v, 16);
+    *reinterpret_cast<float4 *>(at) = w;
+  } else {
+    *reinterpret_cast<C2<T> *>(at) = v;
+  }
+}
+template <typename T>
+__device__ __forceinline__ void reg_convert(C2<T> &v, int sexp) {
+  if constexpr (std::is_same<T, df>::value) {
+    double2 d;
+    memcpy(&d, &v, 16);
+    const df re = to_df(d.x, sexp), im = to_df(d.y, sexp);
+    v = dfc{make_float2(re.h, im.h), make_float2(re.l, im.l)};
+  }
+}
+
+template <typename T>
+__device__ __forceinline__ void reg_unconvert(C2<T> &v, int sexp) {
+  if constexpr (std::is_same<T, df>::value) {
+    const double2 d = make_double2(from_df(df{v.h.x, v.l.x}, sexp), from_df(df{v.h.y, v.l.y}, sexp));
+    memcpy(&v, &d, 16);
+  }
+}
+
+template <typename T, int SIGN, int NF, bool TF>
+__global__ void __launch_bounds__(RegShape<T, NF>::NTH, RegShape<T, NF>::S.minb)
+    fft_reg_kernel(const __grid_constant__ dmg_fft_pass p, const __grid_constant__ dmg_fft_batch bt,
+                   const __grid_constant__ reg_lines lines) {
+  using G = RegShape<T, NF>;
+  constexpr int TL = G::TL, W = G::W, NTH = G::NTH, ES = G::ES, NS = G::S.ns;
+  constexpr bool DFT = std::is_same<T, df>::value;
+  extern __shared__ __align__(16) unsigned char sm[];
+  C2<T> *buf = reinterpret_cast<C2<T> *>(sm);
+  C2<T> *tws = reinterpret_cast<C2<T> *>(sm + G::tw_off(TF));
+  // offsets along t: by transform coordinate (slot order folded in); along t in slot order: by slot, with
+  // the position in the exchange buffer
+  int32_t *tin = reinterpret_cast<int32_t *>(sm + G::tin_off(TF));
+  int32_t *tout = reinterpret_cast<int32_t *>(sm + G::tout_off(TF, SIGN));
+  int2 *sin = reinterpret_cast<int2 *>(tin), *sout = reinterpret_cast<int2 *>(tout);
+  const unsigned char **lptr = reinterpret_cast<const unsigned char **>(sm + G::ptr_off(TF, SIGN));
+  const int tid = threadIdx.x;
+  const bool slot_in = TF && SIGN > 0 && p.perm_in, slot_out = TF && SIGN < 0 && p.perm_out;
+
+  reg_twiddles<T, SIGN, NF, 1>(reinterpret_cast<const C2<T> *>(p.roots), tws, tid);
+  {
+    const int d0 = p.kdim[0], m0 = p.kisz[0] ? p.A[d0] : 1;
+    const int64_t *ti = p.in.tab[d0], *to = p.out.tab[d0];
+    const int64_t i0 = __ldg(ti), o0 = __ldg(to);
+    for (int s = tid; s < NF; s += NTH) {
+      // layout slot s holds line position k of a side in slot order
+      const int k = (p.perm_in || p.perm_out) ? s / p.perm_a + p.perm_b * (s % p.perm_a) : s;
+      const int32_t oi = (int32_t)(__ldg(ti + (int64_t)s * m0) - i0), oo = (int32_t)(__ldg(to + (int64_t)s * m0) - o0);
+      if (slot_in) sin[s] = make_int2((k / G::in_row) * G::in_pitch + k % G::in_row, oi);
+      else tin[p.perm_in ? k : s] = oi;
+      if (slot_out) sout[s] = make_int2((k / G::out_row) * G::out_pitch + k % G::out_row, oo);
+      else tout[p.perm_out ? k : s] = oo;
+    }
+  }
+  __syncthreads();
+
+  const int l = TF ? tid / TL : tid % W, bl = TF ? tid % TL : tid / W;
+  C2<T> *const bx = TF ? buf + l * G::line_pitch() : buf + l;
+  const bool in64 = DFT && p.in_fp64, out64 = DFT && p.out_fp64;
+  // the twiddle's table and its strides along k and y (the order whose neighbouring entries the lanes read)
+  const int td = p.t >> 1;
+  const bool kmaj = !TF && p.kdim[1] == td && !p.kisz[1];
+  const C2<T> *const twt = reinterpret_cast<const C2<T> *>(kmaj ? p.twk[td] : p.twy[td]);
+  const int tw_k = kmaj ? p.A[td] : 1, tw_y = kmaj ? 1 : NF;
+
+  const uint32_t ntiles = (lines.total + W - 1) / W;
+  for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    const uint32_t line = tile * W + l;
+    const bool act = line < lines.total;
+    // the line's place: coordinates per dimension, then its address on each side
+    const unsigned char *src = nullptr;
+    unsigned char *dst = nullptr;
+    int ytw = 0, sexp = 0;
+    if (act) {
+      uint32_t r = line;
+      int x[DMG_FFT_MAXDIM] = {0, 0, 0};
+#pragma unroll
+      for (int i = 0; i < 5; ++i) {
+        if (i < (int)lines.nax) {
+          const reg_axis &ax = lines.ax[i];
+          const uint32_t q = fast_div(r, ax);
+          const int c = (int)(r - q * ax.len);
+          r = q;
+          const int step = c * ax.mul;
+          x[0] += ax.dim == 0 ? step : 0;
+          x[1] += ax.dim == 1 ? step : 0;
+          x[2] += ax.dim == 2 ? step : 0;
+          ytw += ax.isy ? c : 0;
+        }
+      }
+      int64_t ai = p.in.base, ao = p.out.base;
+#pragma unroll
+      for (int d = 0; d < DMG_FFT_MAXDIM; ++d) {
+        if (d < p.ndim) {
+          ai += __ldg(p.in.tab[d] + x[d]);
+          ao += __ldg(p.out.tab[d] + x[d]);
+        }
+      }
+      src = static_cast<const unsigned char *>(bt.src[r]) + ai * ES;
+      dst = static_cast<unsigned char *>(bt.dst[r]) + ao * ES;
+      if (DFT && (in64 || out64)) sexp = __ldg(bt.scale_exp[r]) - 1022;
+    }
+
+    // ---- the first stage's values ----
+    constexpr int R1 = G::R(0), M1 = G::M(0), NB1 = G::NB(0), TR1 = G::TR(0);
+    C2<T> a[TR1 * R1];
+    if (TF && slot_in) {
+      // in slot order through shared memory: lanes run along the slots
+      constexpr int LS = NTH >= NF ? NTH / NF : 1;          // lines at a time
+      constexpr int J = NTH >= NF ? 1 : (NF + NTH - 1) / NTH;  // slots per thread and line
+      constexpr int LI = (W + LS - 1) / LS;
+      __syncthreads();  // the buffer and the pointers of the previous tile have been read
+      if (bl == 0) lptr[l] = src;
+      __syncthreads();
+      const int s0 = NTH >= NF ? tid % NF : tid, l0 = NTH >= NF ? tid / NF : 0;
+      C2<T> v[LI * J];
+#pragma unroll
+      for (int i = 0; i < LI; ++i) {
+        const int lc = l0 + i * LS;
+        const unsigned char *lp = l0 < LS && lc < W ? lptr[lc] : nullptr;
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+          const int s = s0 + j * NTH;
+          v[i * J + j] = C2<T>{};
+          if (lp && (NTH >= NF || NF % NTH == 0 || s < NF)) v[i * J + j] = reg_load<T>(lp + (int64_t)sin[s].y * ES);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < LI; ++i) {
+        const int lc = l0 + i * LS;
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+          const int s = s0 + j * NTH;
+          if (l0 < LS && lc < W && (NTH >= NF || NF % NTH == 0 || s < NF))
+            buf[lc * G::line_pitch() + sin[s].x] = v[i * J + j];
+        }
+      }
+      __syncthreads();
+#pragma unroll
+      for (int tr = 0; tr < TR1; ++tr) {
+        const int b = bl + tr * TL;
+        if (NB1 % TL == 0 || b < NB1) {
+#pragma unroll
+          for (int q = 0; q < R1; ++q) a[tr * R1 + q] = bx[q * G::in_pitch + b];
+        }
+      }
+    } else if (act) {
+#pragma unroll
+      for (int tr = 0; tr < TR1; ++tr) {
+        const int b = bl + tr * TL;
+        if (NB1 % TL == 0 || b < NB1) {
+#pragma unroll
+          for (int q = 0; q < R1; ++q) a[tr * R1 + q] = reg_load<T>(src + (int64_t)tin[b + q * M1] * ES);
+        }
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < TR1 * R1; ++i) a[i] = C2<T>{};
+    }
+    if (in64) {
+#pragma unroll
+      for (int i = 0; i < TR1 * R1; ++i) reg_convert<T>(a[i], sexp);
+    }
+    if (SIGN > 0 && p.twiddle == 2 && act && ytw) {
+#pragma unroll
+      for (int tr = 0; tr < TR1; ++tr) {
+        const int b = bl + tr * TL;
+        if (NB1 % TL == 0 || b < NB1) {
+#pragma unroll
+          for (int q = 0; q < R1; ++q)
+            a[tr * R1 + q] = rmul<T>(a[tr * R1 + q], root_at<T, 1>(twt, (b + q * M1) * tw_k + ytw * tw_y));
+        }
+      }
+    }
+#pragma unroll
+    for (int tr = 0; tr < TR1; ++tr) {
+      const int b = bl + tr * TL;
+      if (NB1 % TL == 0 || b < NB1) reg_butterfly<T, SIGN, NF, 0>(a + tr * R1, tws, 0);
+    }
+
+    // ---- the other stages ----
+    constexpr int RL = G::R(NS - 1), LPL = G::LP(NS - 1), NBL = G::NB(NS - 1), TRL = G::TR(NS - 1);
+    C2<T> y[TRL * RL];
+    reg_exchange<T, SIGN, NF, TF, 1>(a, bx, tws, bl, y);
+    if (SIGN < 0 && p.twiddle == 1 && act && ytw) {
+#pragma unroll
+      for (int tr = 0; tr < TRL; ++tr) {
+        const int b = bl + tr * TL;
+        if (NBL % TL == 0 || b < NBL) {
+#pragma unroll
+          for (int s = 0; s < RL; ++s)
+            y[tr * RL + s] = rmul<T>(y[tr * RL + s], root_at<T, -1>(twt, (b + s * LPL) * tw_k + ytw * tw_y));
+        }
+      }
+    }
+
+    // ---- results to the output layout ----
+    if (out64) {
+#pragma unroll
+      for (int i = 0; i < TRL * RL; ++i) reg_unconvert<T>(y[i], sexp);
+    }
+    if (TF && slot_out) {
+      constexpr int LS = NTH >= NF ? NTH / NF : 1;
+      constexpr int J = NTH >= NF ? 1 : (NF + NTH - 1) / NTH;
+      constexpr int LI = (W + LS - 1) / LS;
+      __syncthreads();
+      if (bl == 0) lptr[l] = dst;
+#pragma unroll
+      for (int tr = 0; tr < TRL; ++tr) {
+        const int b = bl + tr * TL;
+        if (NBL % TL == 0 || b < NBL) {
+#pragma unroll
+          for (int s = 0; s < RL; ++s) bx[s * G::out_pitch + b] = y[tr * RL + s];
+        }
+      }
+      __syncthreads();
+      const int s0 = NTH >= NF ? tid % NF : tid, l0 = NTH >= NF ? tid / NF : 0;
+#pragma unroll
+      for (int j = 0; j < J; ++j) {
+        const int s = s0 + j * NTH;
+        if (l0 < LS && (NTH >= NF || NF % NTH == 0 || s < NF)) {
+          const int2 so = sout[s];
+#pragma unroll
+          for (int i = 0; i < LI; ++i) {
+            const int lc = l0 + i * LS;
+            if (W % LS == 0 || lc < W) {
+              unsigned char *lp = const_cast<unsigned char *>(lptr[lc]);
+              if (lp) reg_store<T>(lp + (int64_t)so.y * ES, buf[lc * G::line_pitch() + so.x]);
+            }
+          }
+        }
+      }
+    } else if (act) {
+#pragma unroll
+      for (int tr = 0; tr < TRL; ++tr) {
+        const int b = bl + tr * TL;
+        if (NBL % TL == 0 || b < NBL) {
+#pragma unroll
+          for (int s = 0; s < RL; ++s) reg_store<T>(dst + (int64_t)tout[b + s * LPL] * ES, y[tr * RL + s]);
+        }
+      }
+    }
+  }
+}
+
+// ---------------------------------------------------------------- launch
+
+template <typename T, int SIGN, int NF, bool TF>
+int launch_reg_k(const dmg_fft_pass &p, const dmg_fft_batch &bt, const reg_lines &lines, cudaStream_t s) {
+  using G = RegShape<T, NF>;
+  constexpr size_t smem = G::smem(TF, SIGN);
+  static_assert((smem + 1024) * G::S.minb <= 233472, "shared memory of the resident blocks");
+  auto k = fft_reg_kernel<T, SIGN, NF, TF>;
+  if (smem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return dmg_error(DMG_ERR_CUDA, "fft pass smem %zu: %s", smem, cudaGetErrorString(e));
+  }
+  int dev = 0, nsm = 0, per_sm = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, G::NTH, smem);
+  if (per_sm < 1) return dmg_error(DMG_ERR_UNSUPPORTED, "fft pass does not fit on an SM (smem %zu)", smem);
+  int64_t grid = (int64_t)nsm * per_sm;
+  const int64_t ntiles = ((int64_t)lines.total + G::W - 1) / G::W;
+  if (grid > ntiles) grid = ntiles;
+  if (grid < 1) return DMG_OK;
+  k<<<(unsigned)grid, G::NTH, smem, s>>>(p, bt, lines);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return dmg_error(DMG_ERR_CUDA, "fft pass launch: %s", cudaGetErrorString(e));
+  return DMG_OK;
+}
+
+// The axes a pass's lines are numbered along: v1, v2, the batch sub-axes (the
+// jobs are what remains of the line number).
+inline reg_lines reg_lines_of(const dmg_fft_pass &p, const dmg_fft_batch &bt) {
+  reg_lines g;
+  memset(&g, 0, sizeof(g));
+  uint64_t total = (uint64_t)bt.count;
+  auto axis = [&](int sub, int len) {
+    total *= (uint64_t)len;
+    if (len <= 1) return;
+    reg_axis &a = g.ax[g.nax++];
+    uint32_t l = 0;
+    while ((1ull << l) < (uint64_t)len) ++l;
+    a.len = (uint32_t)len;
+    a.shift = l;
+    a.magic = (uint32_t)(((1ull << 32) * ((1ull << l) - (uint64_t)len)) / (uint64_t)len + 1);
+    a.dim = sub >> 1;
+    a.mul = (sub & 1) ? p.A[sub >> 1] : 1;
+    a.isy = (sub >> 1) == (p.t >> 1) && !(sub & 1);
+  };
+  if (p.v1 >= 0) axis(p.v1, p.nv1);
+  if (p.v2 >= 0) axis(p.v2, p.nv2);
+  for (int b = 0; b < p.nbatch; ++b) axis(p.bsub[b], p.blen[b]);
+  g.total = (uint32_t)total;
+  return g;
+}
+
+template <typename T, int SIGN, bool TF>
+int launch_reg_form(const dmg_fft_pass &p, const dmg_fft_batch &bt, cudaStream_t s) {
+  const reg_lines g = reg_lines_of(p, bt);
+  switch (p.n) {
+    case 32: return launch_reg_k<T, SIGN, 32, TF>(p, bt, g, s);
+    case 48: return launch_reg_k<T, SIGN, 48, TF>(p, bt, g, s);
+    case 64: return launch_reg_k<T, SIGN, 64, TF>(p, bt, g, s);
+    case 96: return launch_reg_k<T, SIGN, 96, TF>(p, bt, g, s);
+    case 120: return launch_reg_k<T, SIGN, 120, TF>(p, bt, g, s);
+    case 128: return launch_reg_k<T, SIGN, 128, TF>(p, bt, g, s);
+    case 160: return launch_reg_k<T, SIGN, 160, TF>(p, bt, g, s);
+    case 192: return launch_reg_k<T, SIGN, 192, TF>(p, bt, g, s);
+    case 240: return launch_reg_k<T, SIGN, 240, TF>(p, bt, g, s);
+    case 256: return launch_reg_k<T, SIGN, 256, TF>(p, bt, g, s);
+    case 320: return launch_reg_k<T, SIGN, 320, TF>(p, bt, g, s);
+    case 384: return launch_reg_k<T, SIGN, 384, TF>(p, bt, g, s);
+    case 480: return launch_reg_k<T, SIGN, 480, TF>(p, bt, g, s);
+    case 512: return launch_reg_k<T, SIGN, 512, TF>(p, bt, g, s);
+    case 1024: return launch_reg_k<T, SIGN, 1024, TF>(p, bt, g, s);
+    case 2048:
+      if constexpr (std::is_same<T, float>::value) return launch_reg_k<T, SIGN, 2048, TF>(p, bt, g, s);
+    default: return dmg_error(DMG_ERR_ARG, "fft pass: no register schedule for length %d", p.n);
+  }
+}
+
+}  // namespace

@@ -1,0 +1,6 @@
+// FFT passes with lines in registers (double-float arithmetic, forward direction, the form along v1); see fft_reg.cuh.
+#include "fft_reg.cuh"
+
+int dmg_fft_reg_df_fwd_v(const dmg_fft_pass *p, const dmg_fft_batch *b, void *stream) {
+  return launch_reg_form<df, -1, false>(*p, *b, static_cast<cudaStream_t>(stream));
+}

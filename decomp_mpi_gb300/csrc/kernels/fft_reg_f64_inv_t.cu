@@ -1,0 +1,6 @@
+// FFT passes with lines in registers (native FP64 arithmetic, inverse direction, the form along t); see fft_reg.cuh.
+#include "fft_reg.cuh"
+
+int dmg_fft_reg_f64_inv_t(const dmg_fft_pass *p, const dmg_fft_batch *b, void *stream) {
+  return launch_reg_form<double, 1, true>(*p, *b, static_cast<cudaStream_t>(stream));
+}
