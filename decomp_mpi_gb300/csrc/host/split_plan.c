@@ -783,9 +783,9 @@ static int build_passes_split(struct dmg_split_impl *im) {
     axis_letters(p->load_order, lo);
     axis_letters(p->store_order, so);
     pos += snprintf(im->desc + pos, sizeof(im->desc) - pos,
-                    " [t=%d n=%d v1=%d x%d v2=%d x%d tiles=%lld%s in=%s%s out=%s%s%s]", p->t, p->n, p->v1, p->M1, p->v2,
-                    p->M2, (long long)p->ntiles, p->twiddle ? " tw" : "", lo, side_kind(p->sep_in, p->semi_in, p->pair_in), so,
-                    side_kind(p->sep_out, p->semi_out, p->pair_out), reg_name[p->reg]);
+                    " [t=%d n=%d v1=%d x%d v2=%d x%d tiles=%lld%s%s in=%s%s out=%s%s]", p->t, p->n, p->v1, p->M1, p->v2,
+                    p->M2, (long long)p->ntiles, p->twiddle ? " tw" : "", reg_name[p->reg], lo, side_kind(p->sep_in, p->semi_in, p->pair_in), so,
+                    side_kind(p->sep_out, p->semi_out, p->pair_out));
   }
   return DMG_OK;
 }
@@ -864,10 +864,10 @@ static int build_passes_line(struct dmg_split_impl *im) {
     axis_letters(p->load_order, lo);
     axis_letters(p->store_order, so);
     pos += snprintf(im->desc + pos, sizeof(im->desc) - pos,
-                    " [d=%d n=%d v1=%d x%d v2=%d x%d tiles=%lld%s in=%s%s out=%s%s%s]", p->t / 2, p->n,
+                    " [d=%d n=%d v1=%d x%d v2=%d x%d tiles=%lld%s%s in=%s%s out=%s%s]", p->t / 2, p->n,
                     p->v1 >= 0 ? p->v1 / 2 : -1, p->M1, p->v2 >= 0 ? p->v2 / 2 : -1, p->M2, (long long)p->ntiles,
-                    p->perm_out ? " slots" : "", lo, side_kind(p->sep_in, p->semi_in, p->pair_in), so,
-                    side_kind(p->sep_out, p->semi_out, p->pair_out), reg_name[p->reg]);
+                    p->perm_out ? " slots" : "", reg_name[p->reg], lo, side_kind(p->sep_in, p->semi_in, p->pair_in), so,
+                    side_kind(p->sep_out, p->semi_out, p->pair_out));
   }
   return DMG_OK;
 }

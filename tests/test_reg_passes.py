@@ -16,7 +16,7 @@ ARITH = {"fp64": (api.C128, api.ARITH_FP64), "fp32": (api.C64, api.ARITH_FP32), 
 
 
 def _forms(plan):
-    return re.findall(r"n=(\d+) [^\]]*?(?: regs=(\w+))?\]", plan.describe())
+    return re.findall(r"n=(\d+) [^\]]*? tiles=\d+(?: slots| tw)?(?: regs=(\w+))? in=", plan.describe())
 
 
 def _plan(P, spec, **kw):
