@@ -106,8 +106,22 @@ struct dmg_fft_pass {
    * fields above are then unused): both sides separable with the same
    * fastest tile axis and transform-axis offsets that every line shares */
   int32_t reg;
+  const struct dmg_fft_rows *rows; /* (host memory, read when the pass is launched) */
 };
 enum { DMG_FFT_REG_NONE = 0, DMG_FFT_REG_V1 = 1, DMG_FFT_REG_T = 2 };
+
+/* A register pass's thread reads the values b + q n / R1 of its line (q < R1,
+ * R1 the first radix) and writes b + s n / RL (RL the last): where a side's
+ * offsets are the sum of a part in b and a part in q (s), the second part is
+ * the same for every thread and travels here, so that a value costs no table
+ * read.  Offsets in elements from the line's first value, slot order folded
+ * in. */
+#define DMG_FFT_MAXRADIX 32
+struct dmg_fft_rows {
+  int32_t sum_in, sum_out;
+  int32_t r_in, r_out; /* the radices R1 and RL they were made for */
+  int32_t in[DMG_FFT_MAXRADIX], out[DMG_FFT_MAXRADIX];
+};
 
 /* lengths with a register schedule, for values of es bytes */
 static inline int dmg_fft_reg_length(int n, int es) {
@@ -191,6 +205,8 @@ int dmg_fft_pass_launch(const struct dmg_fft_pass *p, int dtype, const void *src
  * complex128 elements of a layout, into *out (which the call first sets to 0). */
 int dmg_fft_maxexp_launch(const struct dmg_fft_layout *lay, int ndim, const int32_t *A, const int32_t *L,
                           const void *src, int32_t *out, void *stream);
+/* First and last radix of a length's register schedule in a form and direction (0: it has none). */
+void dmg_fft_reg_radices(int dtype, int n, int reg, int sign, int *first, int *last);
 /* Shared memory bytes a pass needs. */
 size_t dmg_fft_pass_smem(const struct dmg_fft_pass *p, int dtype);
 #ifdef __cplusplus

@@ -55,6 +55,7 @@ typedef struct {
 
 typedef struct {
   struct dmg_fft_pass p;
+  struct dmg_fft_rows rows; /* register passes */
   int line;                 /* a whole-dimension pass of the lines schedule */
   int in_lay, out_lay;      /* LAY_* */
   int in_buf, out_buf;      /* BUF_* */
@@ -482,6 +483,11 @@ static int t0_rel32(const fft_layout *l, const struct dmg_fft_pass *p) {
   return 1;
 }
 
+/* kernel dtype of a plan's arithmetic */
+static int arith_dtype(const struct dmg_split_impl *im) {
+  return im->arith == DMG_ARITH_FP64 ? 0 : im->arith == DMG_ARITH_FP32 ? 1 : im->arith == DMG_ARITH_DF ? 2 : 3;
+}
+
 /* whether every line of a pass shares a side's offsets along the transform
  * axis (the table's differences from each line's first entry), as int32 */
 static int line_offsets32(const fft_layout *l, const struct dmg_fft_pass *p) {
@@ -512,6 +518,40 @@ static int reg_form(const struct dmg_split_impl *im, const struct dmg_fft_pass *
   if (p->load_order[0] != p->store_order[0] || p->load_order[0] == 2) return DMG_FFT_REG_NONE;
   if (!line_offsets32(li, p) || !line_offsets32(lo, p)) return DMG_FFT_REG_NONE;
   return p->load_order[0] == 0 ? DMG_FFT_REG_T : DMG_FFT_REG_V1;
+}
+
+/* offset of the line's value i on a side */
+static int64_t line_offset(const fft_layout *l, const struct dmg_fft_pass *p, int perm, int i) {
+  const int d = p->kdim[0], step = p->kisz[0] ? p->A[d] : 1;
+  const int64_t s = perm ? (i % p->perm_b) * (int64_t)p->perm_a + i / p->perm_b : i;
+  return l->tab[d][s * step] - l->tab[d][0];
+}
+
+/* Whether the offsets of b + q m (q < r, m = n / r) are a sum of a part in b
+ * and a part in q; fills in the latter. */
+static int rows_sum(const fft_layout *l, const struct dmg_fft_pass *p, int perm, int r, int32_t *out) {
+  const int m = p->n / r;
+  for (int q = 0; q < r; ++q) out[q] = (int32_t)line_offset(l, p, perm, q * m);
+  for (int b = 1; b < m; ++b) {
+    const int64_t ob = line_offset(l, p, perm, b);
+    for (int q = 1; q < r; ++q)
+      if (line_offset(l, p, perm, b + q * m) != ob + out[q]) return 0;
+  }
+  return 1;
+}
+
+/* The register form of a pass (reg_form), with its rows' offsets. */
+static void set_reg_form(const struct dmg_split_impl *im, pass_rec *r, const fft_layout *li, const fft_layout *lo) {
+  r->p.reg = reg_form(im, &r->p, li, lo);
+  memset(&r->rows, 0, sizeof(r->rows));
+  r->p.rows = &r->rows;
+  if (!r->p.reg) return;
+  int first = 0, last = 0;
+  dmg_fft_reg_radices(arith_dtype(im), r->p.n, r->p.reg, r->p.sign, &first, &last);
+  r->rows.r_in = first;
+  r->rows.r_out = last;
+  r->rows.sum_in = rows_sum(li, &r->p, r->p.perm_in, first, r->rows.in);
+  r->rows.sum_out = rows_sum(lo, &r->p, r->p.perm_out, last, r->rows.out);
 }
 
 static void fill_side(struct dmg_fft_layout *fl, const fft_layout *hl, int nd, int64_t base) {
@@ -666,7 +706,7 @@ static int impl_upload(struct dmg_split_impl *im) {
       list[k].p.t0_rel_in = list[k].p.sep_in && t0_rel32(&im->lay[list[k].in_lay], &list[k].p);
       list[k].p.t0_rel_out = list[k].p.sep_out && t0_rel32(&im->lay[list[k].out_lay], &list[k].p);
       const fft_layout *li = &im->lay[list[k].in_lay], *lo = &im->lay[list[k].out_lay];
-      list[k].p.reg = reg_form(im, &list[k].p, li, lo);
+      set_reg_form(im, &list[k], li, lo);
       /* scratch variant: an upper-half side moves to the fixed array */
       pass_rec *sr = dir == 0 ? &im->fwd_s[k] : &im->inv_s[k];
       *sr = list[k];
@@ -682,7 +722,7 @@ static int impl_upload(struct dmg_split_impl *im) {
         lo = &im->lay_s[sr->out_lay];
         fill_side(&sr->p.out, lo, nd, 0);
       }
-      sr->p.reg = reg_form(im, &sr->p, li, lo);
+      set_reg_form(im, sr, li, lo);
     }
   }
   /* a plan small enough for dmg_split_run_noalloc: make the module that
@@ -752,7 +792,7 @@ static int build_passes_split(struct dmg_split_impl *im) {
      * after its transform; the factor is constant along the other dimensions'
      * lines, so it commutes with the remaining stage-1 passes */
     f->p.twiddle = (stage[k] == 1 && K > n1 && im->A[subs[k] / 2] > 1) ? 1 : 0;
-    f->p.reg = reg_form(im, &f->p, &im->lay[in_lay], &im->lay[out_lay]);
+    set_reg_form(im, f, &im->lay[in_lay], &im->lay[out_lay]);
   }
   for (int k = 0; k < K; ++k) {
     /* inverse pass k undoes forward pass K-1-k: it reads what that pass
@@ -771,7 +811,7 @@ static int build_passes_split(struct dmg_split_impl *im) {
     b->line = 0;
     b->p.sign = +1;
     b->p.twiddle = f->p.twiddle ? 2 : 0;
-    b->p.reg = reg_form(im, &b->p, &im->lay[b->in_lay], &im->lay[b->out_lay]);
+    set_reg_form(im, b, &im->lay[b->in_lay], &im->lay[b->out_lay]);
   }
   im->lines = 0;
   int pos = snprintf(im->desc, sizeof(im->desc), "A=[%d,%d,%d] B=[%d,%d,%d] split passes=%d:", im->A[0],
@@ -834,7 +874,7 @@ static int build_passes_line(struct dmg_split_impl *im) {
       f->p.perm_a = im->A[d];
       f->p.perm_b = im->B[d];
     }
-    f->p.reg = reg_form(im, &f->p, &im->lay[f->in_lay], &im->lay[f->out_lay]);
+    set_reg_form(im, f, &im->lay[f->in_lay], &im->lay[f->out_lay]);
   }
   for (int k = 0; k < K; ++k) {
     const pass_rec *f = &im->fwd[K - 1 - k];
@@ -852,7 +892,7 @@ static int build_passes_line(struct dmg_split_impl *im) {
     b->p.perm_in = f->p.perm_out;
     b->p.perm_a = f->p.perm_a;
     b->p.perm_b = f->p.perm_b;
-    b->p.reg = reg_form(im, &b->p, &im->lay[b->in_lay], &im->lay[b->out_lay]);
+    set_reg_form(im, b, &im->lay[b->in_lay], &im->lay[b->out_lay]);
   }
   im->lines = 1;
   int pos = snprintf(im->desc, sizeof(im->desc), "A=[%d,%d,%d] B=[%d,%d,%d] lines passes=%d:", im->A[0],
@@ -891,11 +931,6 @@ static int build_passes(struct dmg_split_impl *im) {
   memset(im->fwd, 0, sizeof(im->fwd));
   memset(im->inv, 0, sizeof(im->inv));
   return use_lines ? build_passes_line(im) : build_passes_split(im);
-}
-
-/* kernel dtype of a plan's arithmetic */
-static int arith_dtype(const struct dmg_split_impl *im) {
-  return im->arith == DMG_ARITH_FP64 ? 0 : im->arith == DMG_ARITH_FP32 ? 1 : im->arith == DMG_ARITH_DF ? 2 : 3;
 }
 
 /* largest exponent of the run's complex128 input, for the double-float scaling */

@@ -1,7 +1,7 @@
 // Entry points of the FFT passes (dispatch by arithmetic) and the exponent
 // pre-pass of double-float runs.  The passes are the execution of
 // runSplitPlan (reference split_fft.c:622-744).
-#include "fft_pass.cuh"
+#include "fft_reg.cuh"
 
 // per-arithmetic launchers (fft_pass_f64.cu, fft_pass_f32.cu, fft_pass_df.cu)
 size_t dmg_fft_pass_smem_f64(const dmg_fft_pass *p);
@@ -99,6 +99,12 @@ __global__ void __launch_bounds__(256) maxexp_rows_kernel(const dmg_fft_layout l
 }
 
 }  // namespace
+
+extern "C" void dmg_fft_reg_radices(int dtype, int n, int reg, int sign, int *first, int *last) {
+  const RegSched s = reg_sched(dtype == 3 ? 1 : dtype, n, reg == DMG_FFT_REG_T, sign > 0);
+  *first = s.ns > 0 ? s.r[0] : 0;
+  *last = s.ns > 0 ? s.r[s.ns - 1] : 0;
+}
 
 extern "C" size_t dmg_fft_pass_smem(const dmg_fft_pass *p, int dtype) {
   return dtype == 0 ? dmg_fft_pass_smem_f64(p)
