@@ -107,6 +107,11 @@ struct dmg_fft_pass {
    * fastest tile axis and transform-axis offsets that every line shares */
   int32_t reg;
   const struct dmg_fft_rows *rows; /* (host memory, read when the pass is launched) */
+  /* the pass runs in the register kernel of any length (fft_gen.cuh), which
+   * takes ranked sides too: process positions along the transform axis and
+   * the rank step between them */
+  int32_t gen;
+  int32_t gen_np_in, gen_rstep_in, gen_np_out, gen_rstep_out;
 };
 enum { DMG_FFT_REG_NONE = 0, DMG_FFT_REG_V1 = 1, DMG_FFT_REG_T = 2 };
 
@@ -207,6 +212,10 @@ int dmg_fft_maxexp_launch(const struct dmg_fft_layout *lay, int ndim, const int3
                           const void *src, int32_t *out, void *stream);
 /* First and last radix of a length's register schedule in a form and direction (0: it has none). */
 void dmg_fft_reg_radices(int dtype, int n, int reg, int sign, int *first, int *last);
+/* Whether the tiled kernel has compile-time stages for a length. */
+int dmg_fft_fixed_length(int n);
+/* Whether the register kernel of any length (p->gen) has room for the pass. */
+int dmg_fft_gen_fits(const struct dmg_fft_pass *p, int dtype);
 /* Shared memory bytes a pass needs. */
 size_t dmg_fft_pass_smem(const struct dmg_fft_pass *p, int dtype);
 #ifdef __cplusplus

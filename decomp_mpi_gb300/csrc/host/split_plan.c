@@ -47,6 +47,7 @@ typedef struct {
   int32_t *rk[DMG_FFT_MAXDIM];
   int64_t *tab[DMG_FFT_MAXDIM];
   int64_t *rstride; /* [ndim][nranks] */
+  int rank_step[DMG_FFT_MAXDIM], positions[DMG_FFT_MAXDIM]; /* rank part = rank_step * process position */
   /* device copies */
   const int64_t *d_tab[DMG_FFT_MAXDIM];
   const int32_t *d_rk[DMG_FFT_MAXDIM];
@@ -168,6 +169,8 @@ static int layout_build(fft_layout *l, Decomp D, long long pitch, const char *wh
     AxisDecomp a = D->dims[d];
     DimDecomp dd = a->decomp;
     int L = dd->coord_size;
+    l->rank_step[d] = a->rank_stride;
+    l->positions[d] = dd->proc_size;
     l->rk[d] = (int32_t *)malloc((size_t)L * sizeof(int32_t));
     l->tab[d] = (int64_t *)malloc((size_t)L * sizeof(int64_t));
     if (!l->rk[d] || !l->tab[d]) return dmg_error(DMG_ERR_NOMEM, "split plan: out of host memory");
@@ -520,6 +523,59 @@ static int reg_form(const struct dmg_split_impl *im, const struct dmg_fft_pass *
   return p->load_order[0] == 0 ? DMG_FFT_REG_T : DMG_FFT_REG_V1;
 }
 
+/* Whether a side suits the register kernel of any length: separable with
+ * shared 32-bit offsets along the line, or ranked with the whole dimension
+ * as the transform axis (the rank then depends on the line and the
+ * coordinate's process position).  Fills in the positions and rank step. */
+static int gen_side(const fft_layout *l, const struct dmg_fft_pass *p, int32_t *np, int32_t *step) {
+  const int d = p->kdim[0];
+  *np = 1;
+  *step = 0;
+  if (!l->ranked) return line_offsets32(l, p);
+  if (p->kisz[0] || p->B[d] != 1) return 0;
+  *np = l->positions[d];
+  *step = l->rank_step[d];
+  for (int x = 0; x < p->n; ++x)
+    if (l->tab[d][x] > INT32_MAX) return 0;
+  return *np <= 64 && *step >= 1;
+}
+
+/* Whether the tiled kernel's compile-time stages are the faster ones for a
+ * pass without a compile-time register form (microseconds at 2^24 values,
+ * tiled against the register kernel of any length):
+ * - double-float passes that convert complex128, except at 8 points and
+ *   where both sides are ranked: 256 points with a ranked output 429 / 498,
+ *   different fastest axes 367 / 500, 16 points along t 254 / 341 (both sides
+ *   ranked 590 / 491, 8 points 731 / 441; without conversions 304 / 233);
+ * - native FP64 from 128 points with different fastest axes or one ranked
+ *   side: 711 / 752, 742 / 777 (64 points 730 / 668, both ranked 882 / 775);
+ * - FP32 16-point lines along t: 133 / 164. */
+static int tiled_faster(const struct dmg_split_impl *im, const struct dmg_fft_pass *p, const fft_layout *li,
+                        const fft_layout *lo, int converts) {
+  if (p->radix_runtime || !dmg_fft_fixed_length(p->n)) return 0;
+  const int mixed = p->load_order[0] != p->store_order[0];
+  if (im->arith == DMG_ARITH_DF) return converts && p->n != 8 && !(li->ranked && lo->ranked);
+  if (im->arith == DMG_ARITH_FP64) return p->n >= 128 && (li->ranked || lo->ranked ? !(li->ranked && lo->ranked) : mixed);
+  return p->n == 16 && p->load_order[0] == 0 && p->store_order[0] == 0;
+}
+
+/* Passes that have no compile-time register form: lengths without a
+ * schedule, radix schedules of the caller's, ranked sides, different fastest
+ * axes.  converts: a double-float pass that reads or writes complex128. */
+static void set_gen_form(const struct dmg_split_impl *im, struct dmg_fft_pass *p, const fft_layout *li,
+                         const fft_layout *lo, int converts) {
+  p->gen = 0;
+  if (p->reg || im->tile_values > 0 || p->n > 2048) return;
+  if (im->arith == DMG_ARITH_TC16 && p->n == 1024 && !p->radix_runtime) return;
+  if (p->sign < 0 ? p->perm_in : p->perm_out) return;
+  if (tiled_faster(im, p, li, lo, converts)) return;
+  if (!gen_side(li, p, &p->gen_np_in, &p->gen_rstep_in) || !gen_side(lo, p, &p->gen_np_out, &p->gen_rstep_out)) return;
+  struct dmg_fft_pass q = *p; /* (the layouts' device form is filled in at the upload) */
+  q.in.ranked = li->ranked;
+  q.out.ranked = lo->ranked;
+  p->gen = dmg_fft_gen_fits(&q, arith_dtype(im));
+}
+
 /* offset of the line's value i on a side */
 static int64_t line_offset(const fft_layout *l, const struct dmg_fft_pass *p, int perm, int i) {
   const int d = p->kdim[0], step = p->kisz[0] ? p->A[d] : 1;
@@ -541,8 +597,10 @@ static int rows_sum(const fft_layout *l, const struct dmg_fft_pass *p, int perm,
 }
 
 /* The register form of a pass (reg_form), with its rows' offsets. */
-static void set_reg_form(const struct dmg_split_impl *im, pass_rec *r, const fft_layout *li, const fft_layout *lo) {
+static void set_reg_form(const struct dmg_split_impl *im, pass_rec *r, const fft_layout *li, const fft_layout *lo,
+                         int converts) {
   r->p.reg = reg_form(im, &r->p, li, lo);
+  set_gen_form(im, &r->p, li, lo, converts);
   memset(&r->rows, 0, sizeof(r->rows));
   r->p.rows = &r->rows;
   if (!r->p.reg) return;
@@ -706,7 +764,7 @@ static int impl_upload(struct dmg_split_impl *im) {
       list[k].p.t0_rel_in = list[k].p.sep_in && t0_rel32(&im->lay[list[k].in_lay], &list[k].p);
       list[k].p.t0_rel_out = list[k].p.sep_out && t0_rel32(&im->lay[list[k].out_lay], &list[k].p);
       const fft_layout *li = &im->lay[list[k].in_lay], *lo = &im->lay[list[k].out_lay];
-      set_reg_form(im, &list[k], li, lo);
+      set_reg_form(im, &list[k], li, lo, k == 0 || k == cnt - 1);
       /* scratch variant: an upper-half side moves to the fixed array */
       pass_rec *sr = dir == 0 ? &im->fwd_s[k] : &im->inv_s[k];
       *sr = list[k];
@@ -722,7 +780,7 @@ static int impl_upload(struct dmg_split_impl *im) {
         lo = &im->lay_s[sr->out_lay];
         fill_side(&sr->p.out, lo, nd, 0);
       }
-      set_reg_form(im, sr, li, lo);
+      set_reg_form(im, sr, li, lo, k == 0 || k == cnt - 1);
     }
   }
   /* a plan small enough for dmg_split_run_noalloc: make the module that
@@ -742,7 +800,7 @@ static const char *side_kind(int sep, int semi, int pair) {
 }
 
 /* lines in registers, and the axis along which lanes run */
-static const char *const reg_name[3] = {"", " regs=v1", " regs=t"};
+static const char *const reg_name[4] = {"", " regs=v1", " regs=t", " regs=any"};
 
 /* A pass's tile axes fastest first in memory, as letters: t the transform
  * axis, a and b the first and second vector axes. */
@@ -792,7 +850,7 @@ static int build_passes_split(struct dmg_split_impl *im) {
      * after its transform; the factor is constant along the other dimensions'
      * lines, so it commutes with the remaining stage-1 passes */
     f->p.twiddle = (stage[k] == 1 && K > n1 && im->A[subs[k] / 2] > 1) ? 1 : 0;
-    set_reg_form(im, f, &im->lay[in_lay], &im->lay[out_lay]);
+    set_reg_form(im, f, &im->lay[in_lay], &im->lay[out_lay], k == 0 || k == K - 1);
   }
   for (int k = 0; k < K; ++k) {
     /* inverse pass k undoes forward pass K-1-k: it reads what that pass
@@ -811,7 +869,7 @@ static int build_passes_split(struct dmg_split_impl *im) {
     b->line = 0;
     b->p.sign = +1;
     b->p.twiddle = f->p.twiddle ? 2 : 0;
-    set_reg_form(im, b, &im->lay[b->in_lay], &im->lay[b->out_lay]);
+    set_reg_form(im, b, &im->lay[b->in_lay], &im->lay[b->out_lay], k == 0 || k == K - 1);
   }
   im->lines = 0;
   int pos = snprintf(im->desc, sizeof(im->desc), "A=[%d,%d,%d] B=[%d,%d,%d] split passes=%d:", im->A[0],
@@ -824,7 +882,7 @@ static int build_passes_split(struct dmg_split_impl *im) {
     axis_letters(p->store_order, so);
     pos += snprintf(im->desc + pos, sizeof(im->desc) - pos,
                     " [t=%d n=%d v1=%d x%d v2=%d x%d tiles=%lld%s%s in=%s%s out=%s%s]", p->t, p->n, p->v1, p->M1, p->v2,
-                    p->M2, (long long)p->ntiles, p->twiddle ? " tw" : "", reg_name[p->reg], lo, side_kind(p->sep_in, p->semi_in, p->pair_in), so,
+                    p->M2, (long long)p->ntiles, p->twiddle ? " tw" : "", reg_name[p->gen ? 3 : p->reg], lo, side_kind(p->sep_in, p->semi_in, p->pair_in), so,
                     side_kind(p->sep_out, p->semi_out, p->pair_out));
   }
   return DMG_OK;
@@ -874,7 +932,7 @@ static int build_passes_line(struct dmg_split_impl *im) {
       f->p.perm_a = im->A[d];
       f->p.perm_b = im->B[d];
     }
-    set_reg_form(im, f, &im->lay[f->in_lay], &im->lay[f->out_lay]);
+    set_reg_form(im, f, &im->lay[f->in_lay], &im->lay[f->out_lay], k == 0 || k == K - 1);
   }
   for (int k = 0; k < K; ++k) {
     const pass_rec *f = &im->fwd[K - 1 - k];
@@ -892,7 +950,7 @@ static int build_passes_line(struct dmg_split_impl *im) {
     b->p.perm_in = f->p.perm_out;
     b->p.perm_a = f->p.perm_a;
     b->p.perm_b = f->p.perm_b;
-    set_reg_form(im, b, &im->lay[b->in_lay], &im->lay[b->out_lay]);
+    set_reg_form(im, b, &im->lay[b->in_lay], &im->lay[b->out_lay], k == 0 || k == K - 1);
   }
   im->lines = 1;
   int pos = snprintf(im->desc, sizeof(im->desc), "A=[%d,%d,%d] B=[%d,%d,%d] lines passes=%d:", im->A[0],
@@ -906,7 +964,7 @@ static int build_passes_line(struct dmg_split_impl *im) {
     pos += snprintf(im->desc + pos, sizeof(im->desc) - pos,
                     " [d=%d n=%d v1=%d x%d v2=%d x%d tiles=%lld%s%s in=%s%s out=%s%s]", p->t / 2, p->n,
                     p->v1 >= 0 ? p->v1 / 2 : -1, p->M1, p->v2 >= 0 ? p->v2 / 2 : -1, p->M2, (long long)p->ntiles,
-                    p->perm_out ? " slots" : "", reg_name[p->reg], lo, side_kind(p->sep_in, p->semi_in, p->pair_in), so,
+                    p->perm_out ? " slots" : "", reg_name[p->gen ? 3 : p->reg], lo, side_kind(p->sep_in, p->semi_in, p->pair_in), so,
                     side_kind(p->sep_out, p->semi_out, p->pair_out));
   }
   return DMG_OK;

@@ -1,0 +1,7 @@
+// FFT passes of any length (double-float arithmetic) writing complex128; see fft_gen.cuh.
+#include "fft_gen.cuh"
+
+int dmg_fft_gen_df_out(const dmg_fft_pass *p, const dmg_fft_batch *b, void *stream, int *taken) {
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  return p->sign > 0 ? launch_gen<df, 1, 2>(*p, *b, s, taken) : launch_gen<df, -1, 2>(*p, *b, s, taken);
+}

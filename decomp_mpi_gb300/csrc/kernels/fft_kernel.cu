@@ -1,7 +1,7 @@
 // Entry points of the FFT passes (dispatch by arithmetic) and the exponent
 // pre-pass of double-float runs.  The passes are the execution of
 // runSplitPlan (reference split_fft.c:622-744).
-#include "fft_reg.cuh"
+#include "fft_gen.cuh"
 
 // per-arithmetic launchers (fft_pass_f64.cu, fft_pass_f32.cu, fft_pass_df.cu)
 size_t dmg_fft_pass_smem_f64(const dmg_fft_pass *p);
@@ -30,6 +30,13 @@ DMG_REG_DECL(f64)
 DMG_REG_DECL(f32)
 DMG_REG_DECL(df)
 #undef DMG_REG_DECL
+// passes of any length with butterflies in registers (fft_gen_*.cu); taken: whether they ran
+int dmg_fft_gen_f64(const dmg_fft_pass *p, const dmg_fft_batch *b, void *stream, int *taken);
+int dmg_fft_gen_f32(const dmg_fft_pass *p, const dmg_fft_batch *b, void *stream, int *taken);
+int dmg_fft_gen_df(const dmg_fft_pass *p, const dmg_fft_batch *b, void *stream, int *taken);
+int dmg_fft_gen_f64_group(const dmg_fft_group *g, void *stream, int *taken);
+int dmg_fft_gen_f32_group(const dmg_fft_group *g, void *stream, int *taken);
+int dmg_fft_gen_df_group(const dmg_fft_group *g, void *stream, int *taken);
 
 namespace {
 
@@ -40,8 +47,12 @@ int64_t reg_line_count(const dmg_fft_pass &p, const dmg_fft_batch &b) {
   return n;
 }
 
+int check_batch_dtype(const dmg_fft_pass &p, const dmg_fft_batch &b, int dtype) {
+  return dtype == 0 ? check_batch<double>(p, b) : dtype == 2 ? check_batch<df>(p, b) : check_batch<float>(p, b);
+}
+
 int launch_reg(const dmg_fft_pass *p, int dtype, const dmg_fft_batch *b, void *stream) {
-  const int st = dtype == 0 ? check_batch<double>(*p, *b) : dtype == 2 ? check_batch<df>(*p, *b) : check_batch<float>(*p, *b);
+  const int st = check_batch_dtype(*p, *b, dtype);
   if (st != DMG_OK) return st;
   const bool t = p->reg == DMG_FFT_REG_T, inv = p->sign > 0;
   using launcher = int (*)(const dmg_fft_pass *, const dmg_fft_batch *, void *);
@@ -106,6 +117,14 @@ extern "C" void dmg_fft_reg_radices(int dtype, int n, int reg, int sign, int *fi
   *last = s.ns > 0 ? s.r[s.ns - 1] : 0;
 }
 
+extern "C" int dmg_fft_fixed_length(int n) { return fixed_length(n); }
+
+extern "C" int dmg_fft_gen_fits(const dmg_fft_pass *p, int dtype) {
+  gen_geom g;
+  return dtype == 0 ? gen_make<double>(*p, 1, 0, &g)
+                    : dtype == 2 ? gen_make<df>(*p, 1, 0, &g) : gen_make<float>(*p, 1, 0, &g);
+}
+
 extern "C" size_t dmg_fft_pass_smem(const dmg_fft_pass *p, int dtype) {
   return dtype == 0 ? dmg_fft_pass_smem_f64(p)
                     : dtype == 1 ? dmg_fft_pass_smem_f32(p)
@@ -123,11 +142,29 @@ extern "C" int dmg_fft_pass_launch_batch(const dmg_fft_pass *p, int dtype, const
     return dmg_error(DMG_ERR_ARG, "fft slot order %d x %d does not match length %d", p->perm_a, p->perm_b, p->n);
   // (the register kernels number lines in 31 bits)
   if (p->reg && dtype >= 0 && dtype <= 3 && reg_line_count(*p, *b) < ((int64_t)1 << 31)) return launch_reg(p, dtype, b, stream);
+  if (p->gen && dtype >= 0 && dtype <= 3) {
+    int taken = 0, st = check_batch_dtype(*p, *b, dtype);
+    if (st == DMG_OK)
+      st = dtype == 0 ? dmg_fft_gen_f64(p, b, stream, &taken)
+                      : dtype == 2 ? dmg_fft_gen_df(p, b, stream, &taken) : dmg_fft_gen_f32(p, b, stream, &taken);
+    if (st != DMG_OK || taken) return st;
+  }
   switch (dtype) {
     case 0: return dmg_fft_pass_launch_f64(p, b, stream);
     case 1: return dmg_fft_pass_launch_f32(p, b, stream);
     case 2: return dmg_fft_pass_launch_df(p, b, stream);
     case 3: return dmg_fft_pass_launch_tc(p, b, stream);
+    default: return dmg_error(DMG_ERR_ARG, "fft dtype %d", dtype);
+  }
+}
+
+static int launch_tiled_group(const dmg_fft_group *g, int dtype, bool inv, void *stream) {
+  switch (dtype) {
+    case 0: return inv ? dmg_fft_pass_f64_inv_group(g, stream) : dmg_fft_pass_f64_fwd_group(g, stream);
+    case 1:
+    case 3:  // the tensor-core form has no runtime-length kernel: its passes run in FP32
+      return inv ? dmg_fft_pass_f32_inv_group(g, stream) : dmg_fft_pass_f32_fwd_group(g, stream);
+    case 2: return inv ? dmg_fft_pass_df_inv_group(g, stream) : dmg_fft_pass_df_fwd_group(g, stream);
     default: return dmg_error(DMG_ERR_ARG, "fft dtype %d", dtype);
   }
 }
@@ -144,19 +181,29 @@ extern "C" int dmg_fft_pass_launch_group(const dmg_fft_group *g, int dtype, void
       return dmg_error(DMG_ERR_ARG, "fft tile %d exceeds %d", p.M1 * p.M2 * p.n, DMG_FFT_TILE_MAX);
     if ((p.perm_in || p.perm_out) && (p.perm_a < 1 || p.perm_b < 1 || (int64_t)p.perm_a * p.perm_b != p.n))
       return dmg_error(DMG_ERR_ARG, "fft slot order %d x %d does not match length %d", p.perm_a, p.perm_b, p.n);
-    const int st = dtype == 0 ? check_batch<double>(p, g->job[j].bt)
-                              : dtype == 2 ? check_batch<df>(p, g->job[j].bt) : check_batch<float>(p, g->job[j].bt);
+    const int st = check_batch_dtype(p, g->job[j].bt, dtype);
     if (st != DMG_OK) return st;
   }
-  const bool inv = sign > 0;
-  switch (dtype) {
-    case 0: return inv ? dmg_fft_pass_f64_inv_group(g, stream) : dmg_fft_pass_f64_fwd_group(g, stream);
-    case 1:
-    case 3:  // the tensor-core form has no runtime-length kernel: its passes run in FP32
-      return inv ? dmg_fft_pass_f32_inv_group(g, stream) : dmg_fft_pass_f32_fwd_group(g, stream);
-    case 2: return inv ? dmg_fft_pass_df_inv_group(g, stream) : dmg_fft_pass_df_fwd_group(g, stream);
-    default: return dmg_error(DMG_ERR_ARG, "fft dtype %d", dtype);
+  if (dtype < 0 || dtype > 3) return dmg_error(DMG_ERR_ARG, "fft dtype %d", dtype);
+  // the passes the any-length register kernel takes run in its launch, the others in the tiled kernel's (the
+  // choice depends on the pass alone, so that every plan's results are those of its own run)
+  int taken[DMG_FFT_MAXGROUP] = {0}, left = 0;
+  const int st = dtype == 0 ? dmg_fft_gen_f64_group(g, stream, taken)
+                            : dtype == 2 ? dmg_fft_gen_df_group(g, stream, taken) : dmg_fft_gen_f32_group(g, stream, taken);
+  if (st != DMG_OK) return st;
+  for (int j = 0; j < g->count; ++j) left += !taken[j];
+  if (left == 0) return DMG_OK;
+  dmg_fft_group *rest = nullptr;
+  if (left < g->count) {
+    rest = static_cast<dmg_fft_group *>(malloc(sizeof(dmg_fft_group)));
+    if (!rest) return dmg_error(DMG_ERR_NOMEM, "grouped fft pass: out of memory");
+    rest->count = 0;
+    for (int j = 0; j < g->count; ++j)
+      if (!taken[j]) rest->job[rest->count++] = g->job[j];
   }
+  const int done = launch_tiled_group(rest ? rest : g, dtype, sign > 0, stream);
+  free(rest);
+  return done;
 }
 
 extern "C" int dmg_fft_pass_launch(const dmg_fft_pass *p, int dtype, const void *src, void *dst, void *stream) {

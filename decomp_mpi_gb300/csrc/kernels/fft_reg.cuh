@@ -285,25 +285,58 @@ __device__ __forceinline__ void rdft8(C2<T> *a) {
     dft8<T, SIGN>(a);
   }
 }
+// a + c v and a + sign i c v for a real constant c: one FMA per component where the arithmetic has it
+template <typename T>
+__device__ __forceinline__ C2<T> mac(C2<T> a, C2<T> v, T c) {
+  if constexpr (std::is_same<T, df>::value) {
+    return add<T>(a, scl<T>(v, c));
+  } else if constexpr (std::is_same<T, float>::value) {
+    return pfma(v, splat(c), a);
+  } else {
+    return make_double2(__fma_rn(c, v.x, a.x), __fma_rn(c, v.y, a.y));
+  }
+}
+template <typename T, int SIGN>
+__device__ __forceinline__ C2<T> mac_rot(C2<T> a, C2<T> v, T c) {
+  if constexpr (std::is_same<T, df>::value) {
+    return add_rot<T, SIGN>(a, scl<T>(v, c));
+  } else {
+    C2<T> r;
+    r.x = fma(SIGN < 0 ? c : -c, v.y, a.x);
+    r.y = fma(SIGN < 0 ? -c : c, v.x, a.y);
+    return r;
+  }
+}
 template <typename T, int SIGN>
 __device__ __forceinline__ void rdft3(C2<T> *a) {
   const C2<T> s = add<T>(a[1], a[2]);
   const C2<T> d = sub<T>(a[1], a[2]);
-  const C2<T> m = sub<T>(a[0], scl<T>(s, cst<T>(K_HALF)));
-  const C2<T> r = scl<T>(d, cst<T>(K_SQRT3_2));
+  const C2<T> m = mac<T>(a[0], s, rneg(cst<T>(K_HALF)));
   a[0] = add<T>(a[0], s);
-  a[1] = add_rot<T, SIGN>(m, r);
-  a[2] = sub_rot<T, SIGN>(m, r);
+  if constexpr (std::is_same<T, df>::value) {
+    const C2<T> r = scl<T>(d, cst<T>(K_SQRT3_2));
+    a[1] = add_rot<T, SIGN>(m, r);
+    a[2] = sub_rot<T, SIGN>(m, r);
+  } else {
+    a[1] = mac_rot<T, SIGN>(m, d, cst<T>(K_SQRT3_2));
+    a[2] = mac_rot<T, -SIGN>(m, d, cst<T>(K_SQRT3_2));
+  }
 }
 template <typename T, int SIGN>
 __device__ __forceinline__ void rdft5(C2<T> *a) {
   const C2<T> b1 = add<T>(a[1], a[4]), b2 = add<T>(a[2], a[3]);
   const C2<T> d1 = sub<T>(a[1], a[4]), d2 = sub<T>(a[2], a[3]);
   const T c1 = cst<T>(K_C72), c2 = cst<T>(K_C144), s1 = cst<T>(K_S72), s2 = cst<T>(K_S144);
-  const C2<T> p1 = add<T>(a[0], add<T>(scl<T>(b1, c1), scl<T>(b2, c2)));
-  const C2<T> p2_ = add<T>(a[0], add<T>(scl<T>(b1, c2), scl<T>(b2, c1)));
-  const C2<T> q1 = add<T>(scl<T>(d1, s1), scl<T>(d2, s2));
-  const C2<T> q2 = sub<T>(scl<T>(d1, s2), scl<T>(d2, s1));
+  C2<T> p1, p2_;
+  if constexpr (std::is_same<T, df>::value) {
+    p1 = add<T>(a[0], add<T>(scl<T>(b1, c1), scl<T>(b2, c2)));
+    p2_ = add<T>(a[0], add<T>(scl<T>(b1, c2), scl<T>(b2, c1)));
+  } else {
+    p1 = mac<T>(mac<T>(a[0], b2, c2), b1, c1);
+    p2_ = mac<T>(mac<T>(a[0], b1, c2), b2, c1);
+  }
+  const C2<T> q1 = mac<T>(scl<T>(d2, s2), d1, s1);
+  const C2<T> q2 = mac<T>(scl<T>(d1, s2), d2, rneg(s1));
   a[0] = add<T>(a[0], add<T>(b1, b2));
   a[1] = add_rot<T, SIGN>(p1, q1);
   a[4] = sub_rot<T, SIGN>(p1, q1);
@@ -497,10 +530,12 @@ struct reg_axis {
   uint32_t len, magic, shift;
   int32_t dim, mul, isy;
 };
-struct reg_lines {
+struct line_axes {
   uint32_t total;  // lines of all jobs
   uint32_t nax;
   reg_axis ax[5];
+};
+struct reg_lines : line_axes {
   dmg_fft_rows rows;
 };
 // r / len for r < 2^31
@@ -509,7 +544,7 @@ __device__ __forceinline__ uint32_t fast_div(uint32_t r, const reg_axis &a) {
 }
 
 // coordinates of a line's first value, the twiddle's y, and its job (returned)
-__device__ __forceinline__ uint32_t line_place(const reg_lines &lines, uint32_t line, int *x, int &y) {
+__device__ __forceinline__ uint32_t line_place(const line_axes &lines, uint32_t line, int *x, int &y) {
   uint32_t r = line;
   x[0] = x[1] = x[2] = 0;
   y = 0;
@@ -1109,8 +1144,8 @@ int launch_reg_k(const dmg_fft_pass &p, const dmg_fft_batch &bt, reg_lines lines
 
 // The axes a pass's lines are numbered along: v1, v2, the batch sub-axes (the
 // jobs are what remains of the line number).
-inline reg_lines reg_lines_of(const dmg_fft_pass &p, const dmg_fft_batch &bt) {
-  reg_lines g;
+inline line_axes line_axes_of(const dmg_fft_pass &p, const dmg_fft_batch &bt) {
+  line_axes g;
   memset(&g, 0, sizeof(g));
   uint64_t total = (uint64_t)bt.count;
   auto axis = [&](int sub, int len) {
@@ -1130,6 +1165,12 @@ inline reg_lines reg_lines_of(const dmg_fft_pass &p, const dmg_fft_batch &bt) {
   if (p.v2 >= 0) axis(p.v2, p.nv2);
   for (int b = 0; b < p.nbatch; ++b) axis(p.bsub[b], p.blen[b]);
   g.total = (uint32_t)total;
+  return g;
+}
+inline reg_lines reg_lines_of(const dmg_fft_pass &p, const dmg_fft_batch &bt) {
+  reg_lines g;
+  memset(&g, 0, sizeof(g));
+  static_cast<line_axes &>(g) = line_axes_of(p, bt);
   if (p.rows) g.rows = *p.rows;
   return g;
 }

@@ -1,5 +1,6 @@
-"""Passes whose lines live in registers (fft_reg.cuh): which passes take that form (CPU), and every length,
-arithmetic and form against the FP64 oracle and the tiled kernel (GPU)."""
+"""Passes whose butterflies run in registers (fft_reg.cuh: lengths with a compile-time schedule; fft_gen.cuh: any
+length, ranked sides, groups): which passes take which form (CPU), and every length, arithmetic and form against
+the FP64 oracle and the tiled kernel (GPU)."""
 import re
 
 import numpy as np
@@ -33,13 +34,15 @@ def test_which_passes_keep_lines_in_registers():
     p.set_tile(1024)  # an explicit tile size keeps the tiled kernel
     assert [f for _, f in _forms(p)] == ["", "", ""]
     p.set_tile(0)
-    p.set_radix(api.RADIX_PLAN8)  # and so does a radix schedule of the caller's
-    assert [f for _, f in _forms(p)] == ["", "", ""]
+    p.set_radix(api.RADIX_PLAN8)  # the caller's radices run in the kernel of any length
+    assert [f for _, f in _forms(p)] == ["any", "any", "any"]
+    p.set_radix(api.RADIX_FIXED)
     # rank buffers too far apart for 32-bit offsets along the line
     far = api.SplitPlan(p.start, 1 << 20, 1 << 40, 1 << 21)
     assert _forms(far) == [("128", ""), ("48", "v1"), ("64", "v1")]
-    # a length without a schedule; 2048 points for 8-byte values only
-    assert _forms(_plan(4, "packed:block(64,2)|block(50,2)|local(128)")) == [("128", "t"), ("50", ""), ("64", "v1")]
+    # a length without a schedule; 2048 points for 8-byte values only (the first double-float pass converts, which
+    # keeps lengths with compile-time tiled stages there unless both sides are ranked)
+    assert _forms(_plan(4, "packed:block(64,2)|block(50,2)|local(128)")) == [("128", "t"), ("50", "any"), ("64", "v1")]
     for dtype, form in ((api.C64, "t"), (api.C128, "")):
         assert _forms(_plan(4, "packed:block(8,2)|block(8,2)|local(2048)", dtype=dtype,
                             schedule=api.SCHEDULE_LINES))[0] == ("2048", form)
@@ -47,10 +50,11 @@ def test_which_passes_keep_lines_in_registers():
     assert _forms(_plan(4, "packed:block(32,2)|block(32,2)|local(1024)", dtype=api.C64,
                         arith=api.ARITH_TC16)) == [("1024", ""), ("32", "v1"), ("32", "v1")]
     # uneven blocks: per-rank strides on the start side
-    assert _forms(_plan(12, "packed:block(64,3)|block(48,4)|local(128)"))[0] == ("128", "")
+    assert _forms(_plan(12, "packed:block(64,3)|block(48,4)|local(128)"))[:2] == [("128", ""), ("48", "any")]
     # Fortran order in memory: the first pass reads along v2 or v1 and writes along t
     fortran = "axes:block(64,2)@1,1|block(64,2)@32,2|local(64)@1024,4"
     assert _forms(_plan(4, fortran))[0] == ("64", "")
+    assert _forms(_plan(4, fortran, dtype=api.C64))[0] == ("64", "any")
     # the split schedule: an interleaved layout's lines share their offsets
     s = _plan(4, "packed:block(1024,2)|block(64,2)|local(64)", schedule=api.SCHEDULE_SPLIT)
     assert ("32", "v1") in _forms(s), s.describe()
@@ -135,3 +139,43 @@ def test_layouts_against_the_tiled_kernel(P, spec, shape, schedule, name, cuda):
     tol = 16 * UNIT[name] * np.log2(np.prod(shape))
     assert _rel(out[0][0][mask], out[1][0][mask]) < tol
     assert _rel(out[0][1], out[1][1]) < 2 * tol
+
+
+ANY = [
+    # (P, start spec, shape): single stages, composite radices, repeated primes, primes without a butterfly
+    # alone, first and last; ranked sides (uneven blocks) on either side, along the lines and along t
+    (1, "packed:local(7)|local(9)|local(2)", (7, 9, 2)),
+    (2, "packed:block(14,2)|local(15)|local(10)", (14, 15, 10)),
+    (4, "packed:block(25,2)|block(35,2)|local(63)", (25, 35, 63)),
+    (6, "packed:block(45,3)|rotate(4,block(40,2))|local(105)", (45, 40, 105)),
+    (7, "packed:local(13)|block(33,7)|local(37)", (13, 33, 37)),
+    (12, "packed:block(30,4)|block(28,3)|local(128)", (30, 28, 128)),
+    (5, "packed:block(243,5)|local(11)|local(6)", (243, 11, 6)),
+    (4, "packed:local(6)|block(10,4)|local(1000)", (6, 10, 1000)),
+    (4, "axes:block(64,2)@1,1|block(50,2)@32,2|local(36)@800,4", (64, 50, 36)),  # Fortran order in memory
+    (3, "packed:block(343,3)", (343,)),
+    (4, "packed:block(101,2)|block(26,2)", (101, 26)),
+]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("radix", [api.RADIX_FIXED, api.RADIX_PLAN8], ids=["own", "plan8"])
+@pytest.mark.parametrize("name", list(ARITH))
+@pytest.mark.parametrize("P,spec,shape", ANY, ids=[str(c[2]) for c in ANY])
+def test_any_length_against_the_oracle(P, spec, shape, name, radix, cuda):
+    import torch
+    plan, dat, work, glob, pitch, wl = _run(cuda, P, spec, shape, name, 5)
+    plan.set_radix(radix)
+    assert any(f == "any" for _, f in _forms(plan)), plan.describe()
+    # (a direct prime DFT of p points sums p products one after the other)
+    tol = 8 * UNIT[name] * (np.log2(np.prod(shape)) + max(q for n in shape for q in range(1, n + 1)
+                                                          if n % q == 0 and all(q % r for r in range(2, q))))
+    st = torch.cuda.current_stream().cuda_stream
+    plan.run(api.FFTW_FORWARD, st)
+    torch.cuda.synchronize()
+    exp, mask = O.split_expected_output(P, spec, glob, wl)
+    assert _rel(work.cpu().numpy()[mask].astype(np.complex128), exp[mask]) < tol
+    plan.run(api.FFTW_BACKWARD, st)
+    torch.cuda.synchronize()
+    back = O.gather_global(P, spec, dat.cpu().numpy().astype(np.complex128), pitch, shape) / np.prod(shape)
+    assert _rel(back, glob) < 2 * tol
