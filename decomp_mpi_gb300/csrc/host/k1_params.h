@@ -25,6 +25,7 @@ struct dmg_k1_side {
   int64_t pitch;                 /* ranked: per-rank pitch in units */
   int32_t nranks;
   int32_t ranked;
+  int32_t np0, rstep0;           /* ranked: process positions along ax0 and the rank step between them */
 };
 
 struct dmg_k1_params {
@@ -39,6 +40,9 @@ struct dmg_k1_params {
   int32_t load_fast;     /* 0: ax0 varies fastest while loading, 1: ax1 */
   int32_t store_fast;    /* same while storing */
   struct dmg_k1_side src, dst;
+  /* direct moves with a ranked side: shared memory of the row-table form
+   * (0: addresses per element) */
+  int32_t rows_smem;
 };
 
 /* Several reshapes in one launch (any sizes and decompositions, each with

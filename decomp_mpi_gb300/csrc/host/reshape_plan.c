@@ -37,6 +37,7 @@ typedef struct {
   int64_t ustride[DMG_MAXAX]; /* uniform memory stride (elements) */
   int64_t *rstride;           /* ranked: [ndim][nranks] memory stride (elements) */
   int64_t max_extent;         /* largest rank extent */
+  int np[DMG_MAXAX], rstep[DMG_MAXAX]; /* process positions per axis, rank part = rstep * position */
 } side_raw;
 
 struct dmg_reshape_impl {
@@ -155,6 +156,8 @@ static int side_build(side_raw *s, Decomp D, const char *side) {
     s->to[i] = (int64_t *)malloc((size_t)L * sizeof(int64_t));
     if (!s->rk[i] || !s->to[i]) return dmg_error(DMG_ERR_NOMEM, "makeReshapePlan: out of memory");
     s->ustride[i] = a->memory_stride;
+    s->np[i] = dd->proc_size;
+    s->rstep[i] = a->rank_stride;
     for (int g = 0; g < L; ++g) {
       int p = dd->rank_offset(dd, g);
       if (p < 0 || p >= dd->proc_size) {
@@ -272,6 +275,9 @@ static int plan_upload(struct dmg_reshape_impl *im) {
     k->ranked = s->ranked;
     k->nranks = s->nranks;
     k->pitch = s->pitch * m;
+    /* (one position on the unit axis, and on a side whose addresses are sums) */
+    k->np0 = s->ranked && im->kp.ax0 < nd ? s->np[im->kp.ax0] : 1;
+    k->rstep0 = s->ranked && im->kp.ax0 < nd ? s->rstep[im->kp.ax0] : 1;
     for (int a = 0; a < na; ++a) {
       int L = im->len[a];
       int64_t *t = h + pos;
@@ -304,6 +310,14 @@ static int plan_upload(struct dmg_reshape_impl *im) {
       k->rstride = dtab + pos;
       pos += (size_t)na * P;
     }
+  }
+  /* row tables for direct moves with a ranked side: an entry per column of the
+   * tile, and per row and position of each side */
+  im->kp.rows_smem = 0;
+  if ((im->s.ranked || im->d.ranked) && im->kp.load_fast == im->kp.store_fast && im->kp.src.rstep0 >= 1 &&
+      im->kp.dst.rstep0 >= 1) {
+    const size_t need = 16 * ((size_t)im->kp.e0 + (size_t)im->kp.e1 * (im->kp.src.np0 + im->kp.dst.np0));
+    if (need <= 36 * 1024) im->kp.rows_smem = (int32_t)need; /* (two of them in three blocks per SM) */
   }
   if (im->fuse_v > 1) {
     int v = im->fuse_v, f = im->kp_fused.ax0;
