@@ -107,6 +107,7 @@ struct dmg_fft_pass {
    * fastest tile axis and transform-axis offsets that every line shares */
   int32_t reg;
   const struct dmg_fft_rows *rows; /* (host memory, read when the pass is launched) */
+  const void *tan;                 /* native FP64: the stages' twiddle entries (dmg_fft_tan_entries) */
   /* the pass runs in the register kernel of any length (fft_gen.cuh), which
    * takes ranked sides too: process positions along the transform axis and
    * the rank step between them */
@@ -212,6 +213,9 @@ int dmg_fft_maxexp_launch(const struct dmg_fft_layout *lay, int ndim, const int3
                           const void *src, int32_t *out, void *stream);
 /* First and last radix of a length's register schedule in a form and direction (0: it has none). */
 void dmg_fft_reg_radices(int dtype, int n, int reg, int sign, int *first, int *last);
+/* Twiddle entries (16 bytes each) of a native FP64 register pass, in its
+ * kernel's order: their number; written to out when it is not NULL. */
+int dmg_fft_tan_entries(int n, int reg, int sign, double *out);
 /* Whether the tiled kernel has compile-time stages for a length. */
 int dmg_fft_fixed_length(int n);
 /* Whether the register kernel of any length (p->gen) has room for the pass. */

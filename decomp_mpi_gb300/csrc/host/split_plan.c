@@ -646,6 +646,15 @@ static int impl_upload(struct dmg_split_impl *im) {
   }
   for (int k = 0; k < im->nfwd; ++k) bytes += align256((size_t)im->fwd[k].p.n * cs);
   for (int d = 0; d < nd; ++d) bytes += 2 * align256((size_t)im->L[d] * cs);
+  if (im->arith == DMG_ARITH_FP64)
+    for (int dir = 0; dir < 2; ++dir)
+      for (int k = 0; k < im->nfwd; ++k) {
+        const struct dmg_fft_pass *p = dir == 0 ? &im->fwd[k].p : &im->inv[k].p;
+        /* (the form is settled below, once the layouts are in place: room for either) */
+        const int a = dmg_fft_tan_entries(p->n, DMG_FFT_REG_V1, p->sign, NULL);
+        const int b = dmg_fft_tan_entries(p->n, DMG_FFT_REG_T, p->sign, NULL);
+        bytes += align256((size_t)(a > b ? a : b) * 16);
+      }
   bytes += 256; /* scale exponent */
   char *host = (char *)calloc(1, bytes + 256);
   if (!host) return dmg_error(DMG_ERR_NOMEM, "split plan: out of host memory for the device tables");
@@ -731,6 +740,18 @@ static int impl_upload(struct dmg_split_impl *im) {
       pos += align256((size_t)im->L[d] * cs);
     }
   }
+  /* native FP64 register passes: their twiddle entries */
+  for (int dir = 0; dir < 2; ++dir)
+    for (int k = 0; k < im->nfwd; ++k) {
+      pass_rec *r = dir == 0 ? &im->fwd[k] : &im->inv[k];
+      r->p.tan = NULL;
+      if (im->arith != DMG_ARITH_FP64) continue;
+      const int form = reg_form(im, &r->p, &im->lay[r->in_lay], &im->lay[r->out_lay]);
+      if (!form) continue;
+      const int n = dmg_fft_tan_entries(r->p.n, form, r->p.sign, (double *)(host + pos));
+      r->p.tan = (char *)dev + pos;
+      pos += align256((size_t)n * 16);
+    }
   im->d_scale = (int32_t *)((char *)dev + pos);
   im->d_status = im->d_scale + 1; /* zero from the upload */
   pos += 256;

@@ -117,6 +117,19 @@ extern "C" void dmg_fft_reg_radices(int dtype, int n, int reg, int sign, int *fi
   *last = s.ns > 0 ? s.r[s.ns - 1] : 0;
 }
 
+extern "C" int dmg_fft_tan_entries(int n, int reg, int sign, double *out) {
+  const RegSched s = reg_sched(0, n, reg == DMG_FFT_REG_T, sign > 0);
+  int at = 0, lp = 1;
+  for (int f = 0; f < s.ns; ++f) {
+    // (as RegShape<double>::tw_per_j; the other stages' entries come from the roots)
+    const int r = s.r[f], per = f == 0 ? 0 : r == 4 || r == 8 ? r : is_pow2(r) ? fma_entries(r) : r - 1;
+    if (out && f > 0 && (r == 4 || r == 8)) tan_table(r, lp, sign, out + 2 * (size_t)at);
+    at += per * lp;
+    lp *= r;
+  }
+  return at;
+}
+
 extern "C" int dmg_fft_fixed_length(int n) { return fixed_length(n); }
 
 extern "C" int dmg_fft_gen_fits(const dmg_fft_pass *p, int dtype) {

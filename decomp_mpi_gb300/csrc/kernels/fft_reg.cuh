@@ -36,6 +36,9 @@
 // 512^3 complex128 double-float 7.95 -> 5.39 ms, native FP64 step (forward,
 // inverse and two reshapes) 38.6 -> 37.1 ms, where the FP64 pipe binds.
 #pragma once
+#include <cmath>
+#include <cstdlib>
+#include <cstring>
 #include "fft_pass.cuh"
 
 namespace {
@@ -75,7 +78,8 @@ enum { AHEAD_NONE = 0, AHEAD_L2 = 1, AHEAD_COPY = 2 };
 //   against 1328 with radices 12 and 8).
 // * Native FP64 is bound by its pipe (86 % busy at 512 points): the odd
 //   radices go first, where they need no twiddles, and the twiddled ones are
-//   powers of two (240: 715 against 645 with radices 16 and 15).
+//   8 and 4, in their form with the fewest operations (240: 785 against 645
+//   with radices 16 and 15; 256: 880 against 815 with 16 and 16).
 __host__ __device__ constexpr RegSched reg_table(int kind, int n, bool t, bool inv) {
   if (kind == 1) {
     switch (n) {
@@ -101,20 +105,20 @@ __host__ __device__ constexpr RegSched reg_table(int kind, int n, bool t, bool i
   if (kind == 0) {
     switch (n) {
       case 32: return {2, {8, 4, 1}, 4, 32, 3, AHEAD_NONE};
-      case 48: return {2, {8, 6, 1}, 8, 16, 4, AHEAD_NONE};
+      case 48: return {2, {6, 8, 1}, 8, 16, 4, AHEAD_NONE};
       case 64: return {2, {8, 8, 1}, 8, 16, 4, AHEAD_NONE};
       case 96: return {2, {12, 8, 1}, 12, 8, 4, AHEAD_NONE};
       case 120: return t ? RegSched{2, {15, 8, 1}, 8, 8, 4, AHEAD_NONE} : RegSched{2, {15, 8, 1}, 15, 8, 4, AHEAD_NONE};
-      case 128: return {2, {16, 8, 1}, 8, 16, 3, AHEAD_NONE};
+      case 128: return {3, {8, 4, 4}, 16, 8, 4, AHEAD_NONE};
       case 160: return {3, {5, 8, 4}, 20, 8, 3, AHEAD_NONE};
       case 192: return {3, {3, 8, 8}, 24, 8, 3, AHEAD_NONE};
       case 240: return {3, {15, 4, 4}, 16, 8, 3, AHEAD_NONE};
-      case 256: return {2, {16, 16, 1}, 16, 8, 3, AHEAD_NONE};
+      case 256: return {3, {8, 8, 4}, 32, 4, 4, AHEAD_NONE};
       case 320: return {3, {20, 4, 4}, 16, 8, 2, AHEAD_NONE};
       case 384: return {3, {6, 8, 8}, 48, 4, 2, AHEAD_NONE};
       case 480: return {3, {15, 8, 4}, 32, 4, 3, AHEAD_NONE};
       case 512: return {3, {8, 8, 8}, 64, 2, 5, AHEAD_NONE};
-      case 1024: return {3, {8, 16, 8}, 64, 4, 2, AHEAD_NONE};
+      case 1024: return {3, {16, 8, 8}, 64, 4, 2, AHEAD_NONE};
       default: return {0, {1, 1, 1}, 1, 1, 1, AHEAD_NONE};
     }
   }
@@ -521,6 +525,111 @@ __device__ __forceinline__ void fma_node(double2 *a, const double2 *tw) {
   }
 }
 
+// Native FP64, twiddled radix 8 and 4 with fewer operations: a twiddle is
+// w_q = i^m c_q (1 + i t_q) with |t_q| <= 1 (its angle within an eighth turn
+// of i^m), so that x'_q = i^m x_q (1 + i t_q) takes two FMAs (the quarter
+// turns are register selects and sign bits), and the scales c_q go into the
+// butterflies' additions, which become FMAs with ratios of scales: 66
+// operations per eight values against 72 in the radix-2 layers above, 22
+// against 24 per four (after Linzer and Feig's FMA forms of the FFT).  The
+// tables come from the host, rounded once: per j the t_q, the ratios, and the
+// quarter turns, two bits a value.  512 points: 24.5 -> 23 operations a value,
+// 720 -> 780 GB/s, and errors 2 % smaller (no doubled differences).
+__device__ __forceinline__ double2 tan_turn(double2 v, double t, unsigned m) {
+  const double p = (m & 1) ? v.y : v.x, r = (m & 1) ? v.x : v.y;
+  // i^m v: the first part negative for m = 1, 2, the second for m = 2, 3
+  const double x = __hiloint2double(__double2hiint(p) ^ (int)(((m ^ (m >> 1)) & 1u) << 31), __double2loint(p));
+  const double y = __hiloint2double(__double2hiint(r) ^ (int)((m >> 1) << 31), __double2loint(r));
+  return make_double2(__fma_rn(-t, y, x), __fma_rn(t, x, y));
+}
+template <int SIGN>
+__device__ __forceinline__ void tan_dft8(double2 *a, const double2 *e) {
+  const unsigned code = (unsigned)__double2loint(e[7].y);
+  const double t[7] = {e[0].x, e[0].y, e[1].x, e[1].y, e[2].x, e[2].y, e[3].x};
+#pragma unroll
+  for (int q = 1; q < 8; ++q) a[q] = tan_turn(a[q], t[q - 1], (code >> (2 * (q - 1))) & 3u);
+  const double rho[4] = {e[3].y, e[4].x, e[4].y, e[5].x};  // c_{q+4} / c_q
+  const double c2 = e[5].y, c31 = e[6].x, c1 = e[6].y, c1h = e[7].x;
+  double2 s[4], d[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    s[q] = mac<double>(a[q], a[q + 4], rho[q]);
+    d[q] = mac<double>(a[q], a[q + 4], -rho[q]);
+  }
+  {
+    const double2 A0 = mac<double>(s[0], s[2], c2), A1 = mac<double>(s[0], s[2], -c2);
+    const double2 B0 = mac<double>(s[1], s[3], c31), B1 = mac<double>(s[1], s[3], -c31);
+    a[0] = mac<double>(A0, B0, c1);
+    a[4] = mac<double>(A0, B0, -c1);
+    a[2] = mac_rot<double, SIGN>(A1, B1, c1);
+    a[6] = mac_rot<double, -SIGN>(A1, B1, c1);
+  }
+  const double2 A0 = mac_rot<double, SIGN>(d[0], d[2], c2), A1 = mac_rot<double, -SIGN>(d[0], d[2], c2);
+  const double2 B0 = mac_rot<double, SIGN>(d[1], d[3], c31), B1 = mac_rot<double, -SIGN>(d[1], d[3], c31);
+  // times the eighth turn: (1 + sign i) / sqrt 2, its scale with c_1
+  const double2 G = add_rot<double, SIGN>(B0, B0), H = add_rot<double, SIGN>(B1, B1);
+  a[1] = mac<double>(A0, G, c1h);
+  a[5] = mac<double>(A0, G, -c1h);
+  a[3] = mac_rot<double, SIGN>(A1, H, c1h);
+  a[7] = mac_rot<double, -SIGN>(A1, H, c1h);
+}
+template <int SIGN>
+__device__ __forceinline__ void tan_dft4(double2 *a, const double2 *e) {
+  const unsigned code = (unsigned)__double2loint(e[3].x);
+  a[1] = tan_turn(a[1], e[0].x, code & 3u);
+  a[2] = tan_turn(a[2], e[0].y, (code >> 2) & 3u);
+  a[3] = tan_turn(a[3], e[1].x, (code >> 4) & 3u);
+  const double c2 = e[1].y, c31 = e[2].x, c1 = e[2].y;
+  const double2 A0 = mac<double>(a[0], a[2], c2), A1 = mac<double>(a[0], a[2], -c2);
+  const double2 B0 = mac<double>(a[1], a[3], c31), B1 = mac<double>(a[1], a[3], -c31);
+  a[0] = mac<double>(A0, B0, c1);
+  a[2] = mac<double>(A0, B0, -c1);
+  a[1] = mac_rot<double, SIGN>(A1, B1, c1);
+  a[3] = mac_rot<double, -SIGN>(A1, B1, c1);
+}
+// Entries of a twiddled stage of radix r after lp points, [entry][j], from
+// the host: for e in order t_1 ... t_{r-1}, then the ratios.
+inline void tan_table(int r, int lp, int sign, double *out) {
+  const long double pi = 3.141592653589793238462643383279502884L;
+  for (int j = 0; j < lp; ++j) {
+    long double c[8], t[8];
+    uint32_t code = 0;
+    for (int q = 0; q < r; ++q) {
+      // angle 2 pi q j / (r lp): quarter turns m and a rest within an eighth
+      const long long num = (long long)q * j, den = (long long)r * lp;
+      const long long m = (8 * num + den) / (2 * den);
+      const long double phi = sign * 2 * pi * ((long double)(4 * num - m * den) / (long double)(4 * den));
+      c[q] = cosl(phi);
+      t[q] = tanl(phi);
+      if (q) code |= (uint32_t)((sign < 0 ? 4 - m % 4 : m) % 4) << (2 * (q - 1));
+    }
+    double bits;
+    const uint64_t word = code;
+    memcpy(&bits, &word, 8);
+    double v[16];
+    int k = 0;
+    for (int q = 1; q < r; ++q) v[k++] = (double)t[q];
+    if (r == 8) {
+      for (int q = 0; q < 4; ++q) v[k++] = (double)(c[q + 4] / c[q]);
+      v[k++] = (double)c[2];
+      v[k++] = (double)(c[3] / c[1]);
+      v[k++] = (double)c[1];
+      v[k++] = (double)(c[1] * sqrtl(0.5L));
+      v[k++] = bits;
+    } else {
+      v[k++] = (double)c[2];
+      v[k++] = (double)(c[3] / c[1]);
+      v[k++] = (double)c[1];
+      v[k++] = bits;
+      v[k++] = 0;
+    }
+    for (int e = 0; e < r; ++e) {
+      out[2 * (e * lp + j)] = v[2 * e];
+      out[2 * (e * lp + j) + 1] = v[2 * e + 1];
+    }
+  }
+}
+
 // ---------------------------------------------------------------- the lines of a pass
 
 // An axis the lines are numbered along: its length (with the constants of a
@@ -618,8 +727,11 @@ struct RegShape {
   }
   static constexpr size_t buf_bytes() { return (size_t)W * (TF ? line_pitch() : line_values()) * ES; }
   // twiddle table entries per j of stage f
+  static constexpr bool tan(int f) { return std::is_same<T, double>::value && f > 0 && (S.r[f] == 4 || S.r[f] == 8); }
   static constexpr bool fma(int f) { return std::is_same<T, double>::value && is_pow2(S.r[f]) && S.r[f] <= 32; }
-  static constexpr int tw_per_j(int f) { return f == 0 ? 0 : fma(f) ? fma_entries(S.r[f]) : S.r[f] - 1; }
+  static constexpr int tw_per_j(int f) {
+    return f == 0 ? 0 : tan(f) ? S.r[f] : fma(f) ? fma_entries(S.r[f]) : S.r[f] - 1;
+  }
   // (8-byte entries lie in pairs, so that one 16-byte read gives a thread two)
   static constexpr int tw_rows(int f) { return ES == 8 ? (tw_per_j(f) + 1) & ~1 : tw_per_j(f); }
   static constexpr int tw_base(int f) { return f <= 1 ? 0 : tw_base(f - 1) + tw_rows(f - 1) * LP(f - 1); }
@@ -653,13 +765,19 @@ struct RegShape {
 
 // ---------------------------------------------------------------- the kernel
 
+// (tan: the pass's host-made entries, at the places of the whole table)
 template <typename T, int SIGN, int NF, bool TF, int F>
-__device__ __forceinline__ void reg_twiddles(const C2<T> *roots, C2<T> *tws, int tid) {
+__device__ __forceinline__ void reg_twiddles(const C2<T> *roots, const C2<T> *tan, C2<T> *tws, int tid) {
   using G = RegShape<T, NF, TF, (SIGN > 0)>;
   if constexpr (F < G::S.ns) {
     constexpr int LP = G::LP(F), R = G::R(F), PJ = G::tw_per_j(F), TS = NF / (LP * R);
     for (int i = tid; i < PJ * LP; i += G::NTH) {
       const int e = i / LP, j = i - e * LP;
+      if constexpr (G::tan(F)) {
+        const int at = G::template tw_at<F>(e, j);
+        tws[at] = __ldg(tan + at);
+        continue;
+      }
       int idx;
       if constexpr (G::fma(F)) {
         // level d, exponent e - 2^{d-1}: w^{R / 2^{d+1}} W_{2^{d+1}}^e
@@ -672,7 +790,7 @@ __device__ __forceinline__ void reg_twiddles(const C2<T> *roots, C2<T> *tws, int
       }
       tws[G::template tw_at<F>(e, j)] = root_at<T, SIGN>(roots, idx % NF);
     }
-    reg_twiddles<T, SIGN, NF, TF, F + 1>(roots, tws, tid);
+    reg_twiddles<T, SIGN, NF, TF, F + 1>(roots, tan, tws, tid);
   }
 }
 
@@ -682,7 +800,13 @@ __device__ __forceinline__ void reg_butterfly(C2<T> *a, const C2<T> *tws, int j)
   using G = RegShape<T, NF, TF, (SIGN > 0)>;
   constexpr int R = G::R(F), LP = G::LP(F);
   const C2<T> *tw = tws + G::template tw_at<F>(0, j);
-  if constexpr (G::fma(F)) {
+  if constexpr (G::tan(F)) {
+    double2 e[R];
+#pragma unroll
+    for (int i = 0; i < R; ++i) e[i] = tw[i * LP];
+    if constexpr (R == 8) tan_dft8<SIGN>(a, e);
+    else tan_dft4<SIGN>(a, e);
+  } else if constexpr (G::fma(F)) {
     if constexpr (F > 0) {
       double2 t[fma_entries(R)];
 #pragma unroll
@@ -851,7 +975,7 @@ __global__ void __launch_bounds__(RegShape<T, NF, TF, (SIGN > 0)>::NTH, RegShape
   const int tid = threadIdx.x;
   const bool slot_in = TF && SIGN > 0 && p.perm_in, slot_out = TF && SIGN < 0 && p.perm_out;
 
-  reg_twiddles<T, SIGN, NF, TF, 1>(reinterpret_cast<const C2<T> *>(p.roots), tws, tid);
+  reg_twiddles<T, SIGN, NF, TF, 1>(reinterpret_cast<const C2<T> *>(p.roots), reinterpret_cast<const C2<T> *>(p.tan), tws, tid);
   {
     const int d0 = p.kdim[0], m0 = p.kisz[0] ? p.A[d0] : 1;
     const int64_t *ti = p.in.tab[d0], *to = p.out.tab[d0];
@@ -1122,6 +1246,7 @@ int launch_reg_k(const dmg_fft_pass &p, const dmg_fft_batch &bt, reg_lines lines
   // offsets made for other radices are no use here: the kernel reads its tables instead
   if (lines.rows.r_in != G::S.r[0]) lines.rows.sum_in = 0;
   if (lines.rows.r_out != G::S.r[G::S.ns - 1]) lines.rows.sum_out = 0;
+  if (std::is_same<T, double>::value && !p.tan) return dmg_error(DMG_ERR_ARG, "fft pass: no twiddle table");
   auto k = fft_reg_kernel<T, SIGN, NF, TF>;
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
