@@ -510,9 +510,11 @@ static int line_offsets32(const fft_layout *l, const struct dmg_fft_pass *p) {
 }
 
 /* The form in which a pass runs with its lines in registers: along t or
- * along v1, whichever is fastest in memory on both sides.  Passes with a
- * tile size or radix schedule of the caller's, ranked sides, or different
- * fastest axes stay with the tiled kernel. */
+ * along v1, whichever is fastest in memory on both sides.  Radix schedules
+ * of the caller's, ranked sides, different fastest axes and lengths without
+ * a schedule go to the kernel of any length (set_gen_form); tile sizes of
+ * the caller's and sides whose offsets differ from line to line to the
+ * tiled one. */
 static int reg_form(const struct dmg_split_impl *im, const struct dmg_fft_pass *p, const fft_layout *li,
                     const fft_layout *lo) {
   if (im->tile_values > 0 || p->radix_runtime || !dmg_fft_reg_length(p->n, im->esize)) return DMG_FFT_REG_NONE;

@@ -1,6 +1,12 @@
-// Batched FFT pass with fused layout change (shared by the translation units
-// fft_pass_{f64,f32,df}{,_inv}{,_mixed}.cu: one per arithmetic, direction and
-// group of lengths).
+// Batched FFT pass with fused layout change, in tiles (shared by the
+// translation units fft_pass_{f64,f32,df}{,_inv}{,_mixed}.cu: one per
+// arithmetic, direction and group of lengths).  The kernels of fft_reg.cuh
+// and fft_gen.cuh, which keep lines in registers, run most passes; this one
+// runs those whose tile the caller chose, whose offsets differ from line to
+// line (two tile axes in one dimension of a layout that is no sum of parts,
+// ranked sides of the split schedule, offsets beyond 32 bits), longer than
+// 2048, on the tensor cores, and those where its compile-time stages are the
+// faster ones (tiled_faster in split_plan.c).
 //
 // One launch transforms every line along one axis and writes the result in
 // another layout: one pass does the work of a reshape (runReshapePlan), a

@@ -1,6 +1,7 @@
 // FFT passes whose lines live in registers: the kernel of every pass whose
 // length has a schedule here, whose sides are separable and whose sides run
-// along the same fastest tile axis (fft_pass.cuh serves the rest).
+// along the same fastest tile axis (fft_gen.cuh serves other lengths, ranked
+// sides and different fastest axes, fft_pass.cuh what is left).
 //
 // A block transforms W whole lines at a time with TL threads per line.  A
 // thread loads the R values of its first butterfly straight from the input
@@ -34,7 +35,7 @@
 // schedule): 1024^3 complex64 FP32 26.1 -> 9.9 ms (7.6 ms at the copy rate);
 // 8 cubes of 240^3 complex64, moved, forward and back, 6.42 -> 2.16 ms;
 // 512^3 complex128 double-float 7.95 -> 5.39 ms, native FP64 step (forward,
-// inverse and two reshapes) 38.6 -> 37.1 ms, where the FP64 pipe binds.
+// inverse and two reshapes) 38.6 -> 34.2 ms, where the FP64 pipe binds.
 #pragma once
 #include <cmath>
 #include <cstdlib>
@@ -321,6 +322,15 @@ __device__ __forceinline__ void rdft3(C2<T> *a) {
     const C2<T> r = scl<T>(d, cst<T>(K_SQRT3_2));
     a[1] = add_rot<T, SIGN>(m, r);
     a[2] = sub_rot<T, SIGN>(m, r);
+  } else if constexpr (std::is_same<T, double>::value) {
+    // The rounding error of sqrt(3)/2 would scale every value of every stage
+    // alike and add up over stages, dimensions and directions (a 432^3 round
+    // trip 7.2e-16, 72^3 5.8e-16): as d - (1 - sqrt(3)/2) d it is an eighth
+    // of that, for two operations more.
+    const T k = -0.133974596215561353236276829247063817;
+    const C2<T> r = mac<T>(d, d, k);
+    a[1] = add_rot<T, SIGN>(m, r);
+    a[2] = sub_rot<T, SIGN>(m, r);
   } else {
     a[1] = mac_rot<T, SIGN>(m, d, cst<T>(K_SQRT3_2));
     a[2] = mac_rot<T, -SIGN>(m, d, cst<T>(K_SQRT3_2));
@@ -588,7 +598,10 @@ __device__ __forceinline__ void tan_dft4(double2 *a, const double2 *e) {
   a[3] = mac_rot<double, -SIGN>(A1, B1, c1);
 }
 // Entries of a twiddled stage of radix r after lp points, [entry][j], from
-// the host: for e in order t_1 ... t_{r-1}, then the ratios.
+// the host: for e in order t_1 ... t_{r-1}, then the ratios.  A scale is that
+// of the rounded t, a ratio that to the rounded scales below it, so that a
+// value's magnitude carries one rounding (48 points: 0.61 -> 0.34 half units
+// rms; a 48^3 round trip 4.33e-16 with every entry rounded by itself).
 inline void tan_table(int r, int lp, int sign, double *out) {
   const long double pi = 3.141592653589793238462643383279502884L;
   for (int j = 0; j < lp; ++j) {
@@ -599,8 +612,8 @@ inline void tan_table(int r, int lp, int sign, double *out) {
       const long long num = (long long)q * j, den = (long long)r * lp;
       const long long m = (8 * num + den) / (2 * den);
       const long double phi = sign * 2 * pi * ((long double)(4 * num - m * den) / (long double)(4 * den));
-      c[q] = cosl(phi);
-      t[q] = tanl(phi);
+      t[q] = (double)tanl(phi);
+      c[q] = 1 / sqrtl(1 + t[q] * t[q]);
       if (q) code |= (uint32_t)((sign < 0 ? 4 - m % 4 : m) % 4) << (2 * (q - 1));
     }
     double bits;
@@ -609,17 +622,19 @@ inline void tan_table(int r, int lp, int sign, double *out) {
     double v[16];
     int k = 0;
     for (int q = 1; q < r; ++q) v[k++] = (double)t[q];
+    const double c1 = (double)c[1], c2 = (double)c[2], c31 = (double)(c[3] / c1);
     if (r == 8) {
-      for (int q = 0; q < 4; ++q) v[k++] = (double)(c[q + 4] / c[q]);
-      v[k++] = (double)c[2];
-      v[k++] = (double)(c[3] / c[1]);
-      v[k++] = (double)c[1];
+      const long double below[4] = {1, c1, c2, (long double)c31 * c1};
+      for (int q = 0; q < 4; ++q) v[k++] = (double)(c[q + 4] / below[q]);
+      v[k++] = c2;
+      v[k++] = c31;
+      v[k++] = c1;
       v[k++] = (double)(c[1] * sqrtl(0.5L));
       v[k++] = bits;
     } else {
-      v[k++] = (double)c[2];
-      v[k++] = (double)(c[3] / c[1]);
-      v[k++] = (double)c[1];
+      v[k++] = c2;
+      v[k++] = c31;
+      v[k++] = c1;
       v[k++] = bits;
       v[k++] = 0;
     }
