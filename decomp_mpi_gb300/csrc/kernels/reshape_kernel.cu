@@ -316,8 +316,10 @@ __device__ __forceinline__ void direct_tile(const dmg_k1_params &p, const U *__r
 // the position and the offset within it; an element then costs three shared
 // reads and two multiply-adds, and the next tile's tables fill while its
 // loads are under way.  250 x 333 x 190 complex128, both sides ranked: 217 ->
-// 120 us (142 without the overlap; its bytes at the copy rate: 75 us); 887 x
-// 682 x 32 int64, both ways: 458 -> 239 us.
+// 110 us (its bytes at the copy rate: 75 us); 996 x 83 x 78 int64, both ways:
+// 175 -> 87 us.  Where a block has one tile nothing hides the tables: they
+// fill in one loop (956 x 27 x 30 int64: 14.4 us per element, 17.4 with a
+// loop per table, 12.4 so).
 constexpr int64_t ROW_ABSENT = INT64_MIN;
 
 template <bool RANKED>
@@ -401,10 +403,14 @@ __device__ __forceinline__ rows_place rows_fill(const dmg_k1_params &p, int64_t 
   w.g1 = t1 * p.e1;
   w.lim0 = min(p.e0, p.len[p.ax0] - w.g0);
   w.lim1 = p.ax1 >= 0 ? min(p.e1, p.len[p.ax1] - w.g1) : 1;
-  for (int i = tid; i < w.lim0; i += NT)
-    cols[i] = make_longlong2(col_entry<SR>(p, p.src, w.g0 + i), col_entry<DR>(p, p.dst, w.g0 + i));
-  for (int i = tid; i < w.lim1 * nps; i += NT) srows[i] = row_entry<SR>(p, p.src, i % nps, w.g1 + i / nps, bc);
-  for (int i = tid; i < w.lim1 * npd; i += NT) drows[i] = row_entry<DR>(p, p.dst, i % npd, w.g1 + i / npd, bc);
+  // (one loop over all entries: the loads of the three tables wait side by side, not one after the other)
+  const int ns = w.lim1 * nps, nd = w.lim1 * npd;
+  for (int i = tid; i < w.lim0 + ns + nd; i += NT) {
+    const int is = i - w.lim0, id = is - ns;
+    if (is < 0) cols[i] = make_longlong2(col_entry<SR>(p, p.src, w.g0 + i), col_entry<DR>(p, p.dst, w.g0 + i));
+    else if (id < 0) srows[is] = row_entry<SR>(p, p.src, is % nps, w.g1 + is / nps, bc);
+    else drows[id] = row_entry<DR>(p, p.dst, id % npd, w.g1 + id / npd, bc);
+  }
   return w;
 }
 // Moves a tile whose tables are filled; meanwhile() runs between its loads and its stores.
@@ -443,11 +449,11 @@ __device__ __forceinline__ void rows_move(const dmg_k1_params &p, const U *__res
     if (da[j] >= 0) dst[da[j]] = v[j];
 }
 
-// resident blocks per SM (the ranked forms spill at the 64 registers of four)
-constexpr int direct_blocks(bool ranked) { return ranked ? 3 : 4; }
+// resident blocks per SM (the ranked forms of 16-byte units spill 250 bytes at the 64 registers of four)
+constexpr int direct_blocks(bool ranked, size_t unit) { return ranked && unit == 16 ? 3 : 4; }
 
 template <typename U, bool SR, bool DR>
-__global__ void __launch_bounds__(NT, direct_blocks(SR || DR)) k1_direct(const dmg_k1_params p, const U *__restrict__ src, U *__restrict__ dst) {
+__global__ void __launch_bounds__(NT, direct_blocks(SR || DR, sizeof(U))) k1_direct(const dmg_k1_params p, const U *__restrict__ src, U *__restrict__ dst) {
   extern __shared__ __align__(16) unsigned char sm[];
   if constexpr (SR || DR) {
     if (p.rows_smem) {
@@ -476,7 +482,7 @@ __global__ void __launch_bounds__(NT, direct_blocks(SR || DR)) k1_direct(const d
 // first_tile), and a block finds the job of each of its tiles.  Every job
 // moves units of the same size and has the same ranked / separable sides.
 template <typename U, bool SR, bool DR>
-__global__ void __launch_bounds__(NT, direct_blocks(SR || DR)) k1_direct_group(const __grid_constant__ dmg_k1_group g) {
+__global__ void __launch_bounds__(NT, direct_blocks(SR || DR, sizeof(U))) k1_direct_group(const __grid_constant__ dmg_k1_group g) {
   extern __shared__ __align__(16) unsigned char sm[];
   for (int64_t tile = blockIdx.x; tile < g.total_tiles; tile += gridDim.x) {
     int j = 0;
