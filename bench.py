@@ -466,7 +466,7 @@ def run_gpu(args):
         "roofline": {"bound": "hbm", "achieved": round(ach64, 1), "peak": peak, "unit": "GB/s",
                      "frac": round(ach64 / peak, 4), "peak_kind": peak_kind,
                      "traffic": ncu_traffic("fft_pass_fp64_512c128"),
-                     "kernel": "fft_pass_kernel<double> (one FP64 FFT pass over the array: 2*N*16 B algorithmic)",
+                     "kernel": "fft_reg_kernel<double> (one FP64 FFT pass over the array: 2*N*16 B algorithmic)",
                      "fp64_pipe": {"achieved_tflops": round(tf64, 3), "peak_tflops": FP64_PEAK_TFLOPS,
                                    "frac": round(tf64 / FP64_PEAK_TFLOPS, 4),
                                    "note": "conventional 5 N log2(n) flops per pass; the pass is bound by the "
@@ -480,7 +480,7 @@ def run_gpu(args):
             "fft_pass_ms": [round(x, 3) for x in ldf], "roundtrip_rel_l2": rtdf,
             "pass_roofline": {"achieved": round(achdf, 1), "peak": peak, "unit": "GB/s", "frac": round(achdf / peak, 4),
                               "traffic": ncu_traffic("fft_pass_512c128"),
-                              "kernel": "fft_pass_kernel<df>"},
+                              "kernel": "fft_reg_kernel<df>"},
             "gpu_launches": df_launches * args.steps * W},
         "e2e": {"value": round(W * flops_step / (e2e_ms * 1e-3) / 1e9, 2), "unit": "GFLOP/s",
                 "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
