@@ -598,22 +598,6 @@ static int rows_sum(const fft_layout *l, const struct dmg_fft_pass *p, int perm,
   return 1;
 }
 
-/* The register form of a pass (reg_form), with its rows' offsets. */
-static void set_reg_form(const struct dmg_split_impl *im, pass_rec *r, const fft_layout *li, const fft_layout *lo,
-                         int converts) {
-  r->p.reg = reg_form(im, &r->p, li, lo);
-  set_gen_form(im, &r->p, li, lo, converts);
-  memset(&r->rows, 0, sizeof(r->rows));
-  r->p.rows = &r->rows;
-  if (!r->p.reg) return;
-  int first = 0, last = 0;
-  dmg_fft_reg_radices(arith_dtype(im), r->p.n, r->p.reg, r->p.sign, &first, &last);
-  r->rows.r_in = first;
-  r->rows.r_out = last;
-  r->rows.sum_in = rows_sum(li, &r->p, r->p.perm_in, first, r->rows.in);
-  r->rows.sum_out = rows_sum(lo, &r->p, r->p.perm_out, last, r->rows.out);
-}
-
 static void fill_side(struct dmg_fft_layout *fl, const fft_layout *hl, int nd, int64_t base) {
   memset(fl, 0, sizeof(*fl));
   for (int d = 0; d < nd; ++d) {
@@ -625,6 +609,53 @@ static void fill_side(struct dmg_fft_layout *fl, const fft_layout *hl, int nd, i
   fl->nranks = hl->nranks;
   fl->ranked = hl->ranked;
   fl->base = base;
+}
+
+/* The rows' offsets of a register pass. */
+static void set_rows(const struct dmg_split_impl *im, pass_rec *r, const fft_layout *li, const fft_layout *lo) {
+  memset(&r->rows, 0, sizeof(r->rows));
+  r->p.rows = &r->rows;
+  if (!r->p.reg) return;
+  int first = 0, last = 0;
+  dmg_fft_reg_radices(arith_dtype(im), r->p.n, r->p.reg, r->p.sign, &first, &last);
+  r->rows.r_in = first;
+  r->rows.r_out = last;
+  r->rows.sum_in = rows_sum(li, &r->p, r->p.perm_in, first, r->rows.in);
+  r->rows.sum_out = rows_sum(lo, &r->p, r->p.perm_out, last, r->rows.out);
+}
+
+/* The register form of a pass (reg_form), with its rows' offsets. */
+static void set_reg_form(const struct dmg_split_impl *im, pass_rec *r, const fft_layout *li, const fft_layout *lo,
+                         int converts) {
+  r->p.reg = reg_form(im, &r->p, li, lo);
+  set_gen_form(im, &r->p, li, lo, converts);
+  set_rows(im, r, li, lo);
+}
+
+/* A pass of dmg_split_run_noalloc: r with its upper-half sides in the fixed
+ * scratch array.  It keeps r's form, so that both runs take the same kernels
+ * and tables (the register forms' twiddle entries are made for r) and give
+ * the same bits.  Where r's offsets along the line are shared and fit 32
+ * bits, so do the scratch array's: its rank pitch is smaller, and a pitch of
+ * at least twice the extent keeps a difference of ranks from making up for
+ * one within a rank.  (A plan too large for the array, which only this
+ * argument's last part leaves out, is refused before it runs.) */
+static void scratch_pass(const struct dmg_split_impl *im, const pass_rec *r, pass_rec *s) {
+  const fft_layout *li = &im->lay[r->in_lay], *lo = &im->lay[r->out_lay];
+  *s = *r;
+  if (s->in_buf == BUF_WORK && s->in_base != 0) {
+    s->in_buf = BUF_SCRATCH;
+    s->in_base = 0;
+    li = &im->lay_s[s->in_lay];
+    fill_side(&s->p.in, li, im->ndim, 0);
+  }
+  if (s->out_buf == BUF_WORK && s->out_base != 0) {
+    s->out_buf = BUF_SCRATCH;
+    s->out_base = 0;
+    lo = &im->lay_s[s->out_lay];
+    fill_side(&s->p.out, lo, im->ndim, 0);
+  }
+  set_rows(im, s, li, lo);
 }
 
 size_t dmg_noalloc_scratch_bytes(void);
@@ -788,22 +819,7 @@ static int impl_upload(struct dmg_split_impl *im) {
       list[k].p.t0_rel_out = list[k].p.sep_out && t0_rel32(&im->lay[list[k].out_lay], &list[k].p);
       const fft_layout *li = &im->lay[list[k].in_lay], *lo = &im->lay[list[k].out_lay];
       set_reg_form(im, &list[k], li, lo, k == 0 || k == cnt - 1);
-      /* scratch variant: an upper-half side moves to the fixed array */
-      pass_rec *sr = dir == 0 ? &im->fwd_s[k] : &im->inv_s[k];
-      *sr = list[k];
-      if (sr->in_buf == BUF_WORK && sr->in_base != 0) {
-        sr->in_buf = BUF_SCRATCH;
-        sr->in_base = 0;
-        li = &im->lay_s[sr->in_lay];
-        fill_side(&sr->p.in, li, nd, 0);
-      }
-      if (sr->out_buf == BUF_WORK && sr->out_base != 0) {
-        sr->out_buf = BUF_SCRATCH;
-        sr->out_base = 0;
-        lo = &im->lay_s[sr->out_lay];
-        fill_side(&sr->p.out, lo, nd, 0);
-      }
-      set_reg_form(im, sr, li, lo, k == 0 || k == cnt - 1);
+      scratch_pass(im, &list[k], dir == 0 ? &im->fwd_s[k] : &im->inv_s[k]);
     }
   }
   /* a plan small enough for dmg_split_run_noalloc: make the module that
@@ -1383,6 +1399,21 @@ double dmg_split_flops(SplitPlan plan) {
   double n = 1;
   for (int i = 0; i < plan->impl->ndim; ++i) n *= plan->impl->L[i];
   return n > 1 ? 5.0 * n * log2(n) : 0.0;
+}
+
+/* The kernel form of each pass of a run (noalloc: of dmg_split_run_noalloc):
+ * 0 tiled, DMG_FFT_REG_* with its lines in registers, 3 the register kernel
+ * of any length.  Returns the number of passes.  Host only. */
+int dmg_split_pass_forms(SplitPlan plan, int direction, int noalloc, int *forms) {
+  const struct dmg_split_impl *im = plan->impl;
+  const pass_rec *list = direction == FFTW_FORWARD ? im->fwd : im->inv;
+  const int cnt = direction == FFTW_FORWARD ? im->nfwd : im->ninv;
+  for (int k = 0; k < cnt; ++k) {
+    pass_rec r = list[k];
+    if (noalloc) scratch_pass(im, &list[k], &r);
+    forms[k] = r.p.gen ? 3 : r.p.reg;
+  }
+  return cnt;
 }
 
 const char *dmg_split_describe(SplitPlan plan) { return plan ? plan->impl->desc : ""; }
