@@ -25,7 +25,7 @@
 // 1575, native FP64 223 / 225 -> 536 / 541; 360 points FP32 540 / 810 -> 1600
 // / 1880, native FP64 379 / 409 -> 482 / 494.  180 x 150 x 105 complex128
 // double-float with uneven blocks 508 -> 267 us; 16 uneven small cubes in one
-// launch per pass, native FP64, 488 -> 330 us.
+// launch per pass, native FP64, 488 -> 354 us.
 #pragma once
 #include "fft_reg.cuh"
 
@@ -101,9 +101,34 @@ __device__ __forceinline__ void rdft9(C2<T> *a) {
     for (int k2 = 0; k2 < 3; ++k2) a[k1 + 3 * k2] = z[k2];
   }
 }
+// Native FP64, eight points: the odd eighth turns as w - (1 - 1/sqrt(2)) w of w = (1 + sign i) v.  The rounding error
+// of 1/sqrt(2) (0.62 units of 2^-53, upwards) would scale a quarter of every stage's values alike; the tiled kernel's
+// partly makes up for that of its sqrt(3)/2 (0.52 downwards), which rdft3 no longer has, and 384 to 1536 points were 3
+// to 4 % further off with it.  So it is 0.09, for four operations more per eight values.
+template <int SIGN>
+__device__ __forceinline__ void gdft8_f64(double2 *a) {
+  double2 e0 = a[0], e1 = a[2], e2 = a[4], e3 = a[6];
+  double2 o0 = a[1], o1 = a[3], o2 = a[5], o3 = a[7];
+  rdft4<double, SIGN>(e0, e1, e2, e3);
+  rdft4<double, SIGN>(o0, o1, o2, o3);
+  const double k = -0.292893218813452475599155637895150961;
+  double2 w1 = add_rot<double, SIGN>(o1, o1), w3 = sub_rot<double, SIGN>(o3, o3);  // (w3: subtracted below)
+  w1 = mac<double>(w1, w1, k);
+  w3 = mac<double>(w3, w3, k);
+  a[0] = cadd(e0, o0);
+  a[4] = csub(e0, o0);
+  a[1] = cadd(e1, w1);
+  a[5] = csub(e1, w1);
+  a[2] = add_rot<double, SIGN>(e2, o2);
+  a[6] = sub_rot<double, SIGN>(e2, o2);
+  a[3] = csub(e3, w3);
+  a[7] = cadd(e3, w3);
+}
 template <typename T, int SIGN, int R>
 __device__ __forceinline__ void gdft(C2<T> *a) {
-  if constexpr (R == 7) {
+  if constexpr (R == 8 && std::is_same<T, double>::value) {
+    gdft8_f64<SIGN>(a);
+  } else if constexpr (R == 7) {
     rdft7<T, SIGN>(a);
   } else if constexpr (R == 9) {
     rdft9<T, SIGN>(a);
@@ -427,38 +452,23 @@ __device__ __forceinline__ void gen_run(const gen_ctx<T> &c, const gen_stage &st
       }
     }
     if constexpr (R > 1) {
-      if constexpr (std::is_same<T, double>::value && (R == 4 || R == 8)) {
-        if (st.lp > 1) {
-          // input twiddles inside the butterflies (the entries fma_node wants)
-          double2 t[R / 2];
-          const int jt = j * ts;
-          if constexpr (R == 8) {
-            t[0] = c.roots[4 * jt];
-            t[1] = c.roots[2 * jt];
-            t[2] = c.roots[jt];
-            t[3] = c.roots[jt + p.n / 8];
-          } else {
-            t[0] = c.roots[2 * jt];
-            t[1] = c.roots[jt];
-          }
-          fma_node<SIGN, R, true, R, 0, 0>(a, t);
-        } else {
-          fma_node<SIGN, R, false, R, 0, 0>(a, nullptr);
+      // (native FP64 multiplies its twiddles separately as well: inside the butterflies, in fma_node's radix-2 layers, they
+      // take 72 operations instead of 84 per eight values, but the layers' doubled differences are rounded twice, and 20
+      // to 1536 points came out 4 to 12 % further off than in the tiled kernel)
+      auto twiddle = [&]() {
+        const C2<T> *w = c.roots;
+#pragma unroll
+        for (int q = 1; q < R; ++q) {
+          w += j * ts;
+          a[q] = rmul<T>(a[q], *w);
         }
-        C2<T> y[R];
-#pragma unroll
-        for (int s = 0; s < R; ++s) y[s] = a[bit_reverse(s, R)];
-#pragma unroll
-        for (int s = 0; s < R; ++s) a[s] = y[s];
+      };
+      // (two paths: as one, with the products predicated, 12 and 16 points took a fifth longer)
+      constexpr bool APART = std::is_same<T, double>::value && (R == 4 || R == 8);
+      if (APART && st.lp == 1) {
+        gdft<T, SIGN, R>(a);
       } else {
-        if (st.lp > 1) {
-          const C2<T> *w = c.roots;
-#pragma unroll
-          for (int q = 1; q < R; ++q) {
-            w += j * ts;
-            a[q] = rmul<T>(a[q], *w);
-          }
-        }
+        if (APART || st.lp > 1) twiddle();
         gdft<T, SIGN, R>(a);
       }
     }
