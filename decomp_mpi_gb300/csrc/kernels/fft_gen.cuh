@@ -516,29 +516,31 @@ __device__ __forceinline__ void gen_run(const gen_ctx<T> &c, const gen_stage &st
   }
 }
 
-// a prime radix without a butterfly: direct DFTs from one buffer to the other
+// A prime radix without a butterfly: direct DFTs from one buffer to the other, an output per thread (with a thread per
+// butterfly, a block's few lines of a long prime left most lanes idle: 512 lines of 1009 points, native FP64, 1430 ms
+// and 651 in the tiled kernel).
 template <typename T, int SIGN>
 __device__ __noinline__ void gen_prime(const gen_ctx<T> &c, const gen_stage &st, const C2<T> *in, C2<T> *out) {
   const gen_geom &g = c.g;
   const int n = c.p.n, r = st.r, ts = n / (st.lp * r), nr = n / r;
-  for (int e = c.tid; e < g.w * st.nb; e += c.nt) {
-    const int l = (int)gen_div((uint32_t)e, st.nb_mul, st.nb_sh), b = e - l * st.nb;
+  const int per = g.w * st.nb;  // butterflies
+  for (int e = c.tid; e < per * r; e += c.nt) {
+    const int s = e / per, i = e - s * per;
+    const int l = (int)gen_div((uint32_t)i, st.nb_mul, st.nb_sh), b = i - l * st.nb;
+    if (c.lin[l * g.in.np].x == 0) continue;  // past the last line
     const int j = (int)gen_div((uint32_t)b, st.m_mul, st.m_sh), k = b - j * st.m;
     const C2<T> *x = in + (j * st.pin + k) * g.s1 + l * g.s2;
-    C2<T> *y = out + (j * st.pout + k) * g.s1 + l * g.s2;
-    for (int s = 0; s < r; ++s) {
-      C2<T> acc = x[0];
-      int tw = 0, ro = 0;  // j q ts, (q s mod r) n / r
-      for (int q = 1; q < r; ++q) {
-        tw += j * ts;
-        ro += s * nr;
-        if (ro >= n) ro -= n;
-        C2<T> v = x[q * st.m * g.s1];
-        if (j) v = rmul<T>(v, c.roots[tw]);
-        acc = add<T>(acc, rmul<T>(v, c.roots[ro]));
-      }
-      y[s * st.lp * st.pout * g.s1] = acc;
+    C2<T> acc = x[0];
+    int tw = 0, ro = 0;  // j q ts, (q s mod r) n / r
+    for (int q = 1; q < r; ++q) {
+      tw += j * ts;
+      ro += s * nr;
+      if (ro >= n) ro -= n;
+      C2<T> v = x[q * st.m * g.s1];
+      if (j) v = rmul<T>(v, c.roots[tw]);
+      acc = add<T>(acc, rmul<T>(v, c.roots[ro]));
     }
+    out[(j * st.pout + k) * g.s1 + l * g.s2 + s * st.lp * st.pout * g.s1] = acc;
   }
 }
 
