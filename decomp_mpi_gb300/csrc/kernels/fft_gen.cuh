@@ -747,14 +747,12 @@ inline int64_t gen_lines_of(const dmg_fft_pass &p, const dmg_fft_batch &bt) {
 
 template <typename K>
 int gen_blocks(K k, int nt, size_t smem, int64_t *blocks) {
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return dmg_error(DMG_ERR_CUDA, "fft pass smem %zu: %s", smem, cudaGetErrorString(e));
-  }
   int dev = 0, nsm = 0, per_sm = 0;
+  cudaError_t e = allow_smem(k, smem);
+  if (e == cudaSuccess) e = resident_blocks(k, nt, smem, &per_sm);
+  if (e != cudaSuccess) return dmg_error(DMG_ERR_CUDA, "fft pass smem %zu: %s", smem, cudaGetErrorString(e));
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, nt, smem);
   if (per_sm < 1) return dmg_error(DMG_ERR_UNSUPPORTED, "fft pass does not fit on an SM (smem %zu)", smem);
   *blocks = (int64_t)nsm * per_sm;
   return DMG_OK;

@@ -63,6 +63,7 @@
 #include <type_traits>
 #include "../host/dmg_internal.h"
 #include "../host/fft_params.h"
+#include "smem_limit.cuh"
 #include "tc_sm100.cuh"
 
 namespace {
@@ -1225,6 +1226,7 @@ struct PassConsts {
   uint32_t tc_taddr;
   int tc_fail;
 };
+constexpr size_t PASS_STATIC = (sizeof(PassConsts) + 127) & ~(size_t)127;  // the kernels' static shared memory at most
 
 __device__ __forceinline__ void tile_digits(const int *rad, int nd, int64_t t, int *dig) {
   for (int i = 0; i < nd; ++i) {
@@ -2107,14 +2109,12 @@ int launch_group(dmg_fft_group g, cudaStream_t s) {
     tiles += g.job[j].p.ntiles * g.job[j].bt.count;
   }
   auto k = fft_pass_group_kernel<T, SIGN>;
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return dmg_error(DMG_ERR_CUDA, "grouped fft pass smem %zu: %s", smem, cudaGetErrorString(e));
-  }
   int dev = 0, nsm = 0, per_sm = 0;
+  cudaError_t es = allow_smem(k, smem, PASS_STATIC);
+  if (es == cudaSuccess) es = resident_blocks(k, NT, smem, &per_sm);
+  if (es != cudaSuccess) return dmg_error(DMG_ERR_CUDA, "grouped fft pass smem %zu: %s", smem, cudaGetErrorString(es));
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, NT, smem);
   if (per_sm < 1) return dmg_error(DMG_ERR_UNSUPPORTED, "grouped fft pass does not fit on an SM (smem %zu)", smem);
   const int64_t budget = (int64_t)nsm * per_sm;
   int64_t first = 0;
@@ -2137,14 +2137,12 @@ template <typename T, int SIGN, int NF, bool TC = false>
 int launch_k(const dmg_fft_pass &p, const dmg_fft_batch &bt, cudaStream_t s) {
   const size_t smem = smem_layout<T>(p, NF > 0, TC).total;
   auto k = fft_pass_kernel<T, SIGN, NF, TC>;
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return dmg_error(DMG_ERR_CUDA, "fft pass smem %zu: %s", smem, cudaGetErrorString(e));
-  }
   int dev = 0, nsm = 0, per_sm = 0;
+  cudaError_t es = allow_smem(k, smem, PASS_STATIC);
+  if (es == cudaSuccess) es = resident_blocks(k, NT, smem, &per_sm);
+  if (es != cudaSuccess) return dmg_error(DMG_ERR_CUDA, "fft pass smem %zu: %s", smem, cudaGetErrorString(es));
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, NT, smem);
   if (per_sm < 1) return dmg_error(DMG_ERR_UNSUPPORTED, "fft pass does not fit on an SM (smem %zu)", smem);
   if constexpr (TC) {
     // the occupancy query answers one block per SM for kernels that allocate tensor memory; two blocks of

@@ -1263,14 +1263,12 @@ int launch_reg_k(const dmg_fft_pass &p, const dmg_fft_batch &bt, reg_lines lines
   if (lines.rows.r_out != G::S.r[G::S.ns - 1]) lines.rows.sum_out = 0;
   if (std::is_same<T, double>::value && !p.tan) return dmg_error(DMG_ERR_ARG, "fft pass: no twiddle table");
   auto k = fft_reg_kernel<T, SIGN, NF, TF>;
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return dmg_error(DMG_ERR_CUDA, "fft pass smem %zu: %s", smem, cudaGetErrorString(e));
-  }
   int dev = 0, nsm = 0, per_sm = 0;
+  cudaError_t es = allow_smem(k, smem);
+  if (es == cudaSuccess) es = resident_blocks(k, G::NTH, smem, &per_sm);
+  if (es != cudaSuccess) return dmg_error(DMG_ERR_CUDA, "fft pass smem %zu: %s", smem, cudaGetErrorString(es));
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, G::NTH, smem);
   if (per_sm < 1) return dmg_error(DMG_ERR_UNSUPPORTED, "fft pass does not fit on an SM (smem %zu)", smem);
   int64_t grid = (int64_t)nsm * per_sm;
   const int64_t ntiles = ((int64_t)lines.total + G::W - 1) / G::W;

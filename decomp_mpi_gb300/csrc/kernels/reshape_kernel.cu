@@ -20,6 +20,7 @@
 #include <cstdio>
 #include "../host/dmg_internal.h"
 #include "../host/k1_params.h"
+#include "smem_limit.cuh"
 
 namespace {
 
@@ -503,17 +504,28 @@ __global__ void __launch_bounds__(NT, direct_blocks(SR || DR, sizeof(U))) k1_dir
   }
 }
 
+// SMs, and blocks of a launch per SM (fixed: static shared memory at most).
+template <typename K>
+int k1_residency(K kern, size_t smem, size_t fixed, int *nsm, int *per_sm) {
+  int dev = 0;
+  cudaError_t e = allow_smem(kern, smem, fixed);
+  if (e == cudaSuccess) e = resident_blocks(kern, NT, smem, per_sm);
+  if (e != cudaSuccess) return dmg_error(DMG_ERR_CUDA, "reshape kernel smem %zu: %s", smem, cudaGetErrorString(e));
+  if (*per_sm < 1) return dmg_error(DMG_ERR_UNSUPPORTED, "reshape kernel does not fit on an SM (smem %zu)", smem);
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(nsm, cudaDevAttrMultiProcessorCount, dev);
+  return DMG_OK;
+}
+
 template <typename U, bool SR, bool DR>
 int launch_direct_group(const dmg_k1_group &g, cudaStream_t stream) {
   auto kern = k1_direct_group<U, SR, DR>;
   size_t smem = 0;
   if (SR || DR)
     for (int j = 0; j < g.count; ++j) smem = (size_t)g.job[j].p.rows_smem > smem ? (size_t)g.job[j].p.rows_smem : smem;
-  int dev = 0, nsm = 0, per_sm = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NT, smem);
-  if (per_sm < 1) per_sm = 1;
+  int nsm = 0, per_sm = 0;
+  const int st = k1_residency(kern, smem, 0, &nsm, &per_sm);
+  if (st != DMG_OK) return st;
   int64_t grid = (int64_t)nsm * per_sm;
   if (grid > g.total_tiles) grid = g.total_tiles;
   if (grid < 1) return DMG_OK;
@@ -536,15 +548,9 @@ template <typename U, bool SR, bool DR>
 int launch_direct(const dmg_k1_params &p, const void *src, void *dst, cudaStream_t stream) {
   auto kern = k1_direct<U, SR, DR>;
   const size_t smem = SR || DR ? 2 * (size_t)p.rows_smem : 0;
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return dmg_error(DMG_ERR_CUDA, "reshape kernel smem attribute: %s", cudaGetErrorString(e));
-  }
-  int dev = 0, nsm = 0, per_sm = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NT, smem);
-  if (per_sm < 1) per_sm = 1;
+  int nsm = 0, per_sm = 0;
+  const int st = k1_residency(kern, smem, 0, &nsm, &per_sm);
+  if (st != DMG_OK) return st;
   int64_t grid = (int64_t)nsm * per_sm;
   if (grid > p.ntiles) grid = p.ntiles;
   if (grid < 1) return DMG_OK;
@@ -560,15 +566,9 @@ int launch_typed(const dmg_k1_params &p, const void *src, void *dst, cudaStream_
   const size_t tilebytes = (sizeof(U) * (size_t)p.e1 * (p.e0 + 1) + 15) & ~size_t(15);
   const size_t smem = tilebytes + (size_t)(p.e0 + p.e1) * 2 * (sizeof(int64_t) + sizeof(int32_t));
   auto kern = k1_permute<U, SR, DR>;
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return dmg_error(DMG_ERR_CUDA, "reshape kernel smem attribute: %s", cudaGetErrorString(e));
-  }
-  int dev = 0, nsm = 0, per_sm = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NT, smem);
-  if (per_sm < 1) per_sm = 1;
+  int nsm = 0, per_sm = 0;
+  const int st = k1_residency(kern, smem, 1024, &nsm, &per_sm);
+  if (st != DMG_OK) return st;
   int64_t grid = (int64_t)nsm * per_sm;
   if (grid > p.ntiles) grid = p.ntiles;
   if (grid < 1) return DMG_OK;
