@@ -1557,12 +1557,14 @@ int dmg_split_batch_launches(SplitPlan plan, int direction, int count) {
 
 /* ---------------------------------------------------------------- grouped run */
 
-_Static_assert(DMG_SPLIT_MAXGROUP == DMG_FFT_MAXGROUP, "a group is one launch per pass");
+_Static_assert(DMG_SPLIT_MAXGROUP == DMG_FFT_MAXGROUP, "a group fits the launches of a pass");
 
 /* The k-th passes of several plans (any sizes, decompositions and pass
- * counts) in one launch each: plan i's pass k reads what its pass k-1 wrote
- * in the launch before, on the same stream.  Every plan runs its passes with
- * the runtime stages of its radix schedule, so it must have one
+ * counts) together, in one launch of the register kernel of any length and,
+ * where a plan's pass is not one of its (dmg_fft_pass.gen), one of the tiled
+ * kernel's runtime stages: plan i's pass k reads what its pass k-1 wrote
+ * in the launches before, on the same stream.  Every plan runs its passes
+ * with the radices of its runtime schedule, so it must have one
  * (DMG_RADIX_PLAN8 or DMG_RADIX_PLAN4); its results are then the bits of
  * dmg_split_run on the same plan.  own_buffers: the plans' dat and workspace
  * are the arrays (else the caller lists them). */
@@ -1670,19 +1672,34 @@ int dmg_split_run_group_batch(int count, SplitPlan const *plans, const int *njob
   return group_run(count, plans, njobs, dats, works, scales, direction, stream);
 }
 
+/* whether the register kernel of any length takes a pass over one array (launch_gen_group's rule) */
+static int pass_in_gen_launch(const struct dmg_fft_pass *p) {
+  int64_t lines = (int64_t)p->nv1 * p->nv2;
+  for (int b = 0; b < p->nbatch; ++b) lines *= p->blen[b];
+  return p->gen && lines < ((int64_t)1 << 31);
+}
+
 int dmg_split_group_launches(int count, SplitPlan const *plans, int direction) {
   if (!plans || group_check(count, plans, direction, 1, "dmg_split_group_launches") != DMG_OK) return 0;
-  int most = 0, pre = 0;
+  int most = 0, launches = 0;
   for (int i = 0; i < count; ++i) {
     const struct dmg_split_impl *im = plans[i]->impl;
     const int cnt = direction == FFTW_FORWARD ? im->nfwd : im->ninv;
     if (cnt > most) most = cnt;
-    if (im->arith == DMG_ARITH_DF) pre += 1; /* the exponent pre-pass, per plan */
+    if (im->arith == DMG_ARITH_DF) launches += 1; /* the exponent pre-pass, per plan */
   }
-  return most + pre;
+  /* the k-th passes: those of the register kernel of any length in one launch, the others in the tiled kernel's */
+  for (int k = 0; k < most; ++k) {
+    int in[2] = {0, 0};
+    for (int i = 0; i < count; ++i) {
+      const struct dmg_split_impl *im = plans[i]->impl;
+      const int cnt = direction == FFTW_FORWARD ? im->nfwd : im->ninv;
+      if (k < cnt) in[pass_in_gen_launch(direction == FFTW_FORWARD ? &im->fwd[k].p : &im->inv[k].p)] = 1;
+    }
+    launches += in[0] + in[1];
+  }
+  return launches;
 }
-
-
 
 /* ---------------------------------------------------------------- no-allocation run */
 

@@ -197,9 +197,13 @@ int dmg_split_batch_launches(SplitPlan plan, int direction, int count);
 #define DMG_SPLIT_MAXGROUP 16
 /** runSplitPlan on up to DMG_SPLIT_MAXGROUP different plans (any sizes,
  * decompositions and pass counts; no counterpart in the reference), each on
- * its own dat and workspace: the k-th passes of all plans share one launch,
- * so a group of small transforms takes as many pass launches as its longest
- * plan has passes.  Every plan must have a runtime radix schedule
+ * its own dat and workspace: the k-th passes of all plans run together, in
+ * one launch of the register kernel of any length and, where some of them
+ * are not passes of that kernel's (longer than 2048 points, ranked sides in
+ * the split schedule, a tile size of the caller's), a second one of the tiled
+ * kernel.  A group of small transforms so takes as many pass launches as its
+ * longest plan has passes, at most twice that
+ * (dmg_split_group_launches counts them).  Every plan must have a runtime radix schedule
  * (DMG_RADIX_PLAN8 or DMG_RADIX_PLAN4) and the same arithmetic; the results
  * are the bits of runSplitPlan on each plan.  Buffers of different plans
  * must not overlap. */
@@ -210,7 +214,9 @@ int dmg_split_run_group(int count, SplitPlan const *plans, int direction, void *
  * plan.  The plans' own dat and workspace are not used. */
 int dmg_split_run_group_batch(int count, SplitPlan const *plans, const int *njobs, void *const *dats,
                               void *const *works, int *const *scales, int direction, void *stream);
-/** Kernel launches of one dmg_split_run_group call (0 if the group is invalid). */
+/** Kernel launches of one dmg_split_run_group call (0 if the group is invalid),
+ * as its plans stand: one or two for each pass, and the exponent pre-pass of
+ * every double-float plan. */
 int dmg_split_group_launches(int count, SplitPlan const *plans, int direction);
 /** Select the pass schedule (no counterpart in the reference). */
 int dmg_split_set_schedule(SplitPlan plan, int schedule);
