@@ -524,6 +524,8 @@ __device__ __noinline__ void gen_prime(const gen_ctx<T> &c, const gen_stage &st,
   const gen_geom &g = c.g;
   const int n = c.p.n, r = st.r, ts = n / (st.lp * r), nr = n / r;
   const int per = g.w * st.nb;  // butterflies
+  // (the input twiddle and the DFT's root are one root of n: a product a value, half of what two take; 1331 points,
+  // 2048 lines, native FP64: 1717 us with two products, 1506 in the tiled kernel, 1020 so)
   for (int e = c.tid; e < per * r; e += c.nt) {
     const int s = e / per, i = e - s * per;
     const int l = (int)gen_div((uint32_t)i, st.nb_mul, st.nb_sh), b = i - l * st.nb;
@@ -531,14 +533,12 @@ __device__ __noinline__ void gen_prime(const gen_ctx<T> &c, const gen_stage &st,
     const int j = (int)gen_div((uint32_t)b, st.m_mul, st.m_sh), k = b - j * st.m;
     const C2<T> *x = in + (j * st.pin + k) * g.s1 + l * g.s2;
     C2<T> acc = x[0];
-    int tw = 0, ro = 0;  // j q ts, (q s mod r) n / r
+    const int step = j * ts + s * nr;  // (each below n, step q = j q ts + q s n / r)
+    int ro = 0;
     for (int q = 1; q < r; ++q) {
-      tw += j * ts;
-      ro += s * nr;
+      ro += step;
       if (ro >= n) ro -= n;
-      C2<T> v = x[q * st.m * g.s1];
-      if (j) v = rmul<T>(v, c.roots[tw]);
-      acc = add<T>(acc, rmul<T>(v, c.roots[ro]));
+      acc = add<T>(acc, rmul<T>(x[q * st.m * g.s1], c.roots[ro]));
     }
     out[(j * st.pout + k) * g.s1 + l * g.s2 + s * st.lp * st.pout * g.s1] = acc;
   }

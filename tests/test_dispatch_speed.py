@@ -54,3 +54,10 @@ def _not_slower(cuda, spec, shape, name):
 @pytest.mark.parametrize("shape", [(211,), (13,), (37, 64), (211, 48), (48, 211), (66, 66, 66)], ids=str)
 def test_direct_primes(shape, name, cuda):
     _not_slower(cuda, "packed:" + "|".join("local(%d)" % n for n in shape), shape, name)
+
+
+
+@pytest.mark.parametrize("name", list(ARITH))
+@pytest.mark.parametrize("shape", [(1331, 512), (512, 1331), (143, 1024)], ids=str)
+def test_twiddled_primes(shape, name, cuda):
+    _not_slower(cuda, "packed:" + "|".join("local(%d)" % n for n in shape), shape, name)
