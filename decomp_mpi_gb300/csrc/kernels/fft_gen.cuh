@@ -160,6 +160,7 @@ __device__ __forceinline__ void gdft(C2<T> *a) {
 // for short lines (more of them in different phases, less to wait for at a
 // barrier), in larger ones where a line needs the room.
 constexpr int GEN_MAXNT = 512;
+constexpr int GEN_SMS = 152;  // GB300's (the geometry is also made where there is no device to ask)
 template <typename T>
 constexpr int gen_per_thread() {
   return std::is_same<T, float>::value ? 16 : 8;
@@ -307,10 +308,23 @@ bool gen_make(const dmg_fft_pass &p, int64_t lines, int nt, gen_geom *g, int con
   int w = g->nt * gen_per_thread<T>() / n;
   if (w < 1) w = 1;
   // (enough blocks for every SM where that leaves a warp of butterflies each)
-  while (w > 1 && (lines + w - 1) / w < 304 && (w / 2) * n >= 32 * gen_per_thread<T>()) w /= 2;
+  while (w > 1 && (lines + w - 1) / w < 2 * GEN_SMS && (w / 2) * n >= 32 * gen_per_thread<T>()) w /= 2;
   if (w >= 8) w &= ~3;
-  for (;; --w) {
-    if (w < 1) return false;
+  // and, with more blocks than SMs, the threads for the lines that are left, as long as their block fits (in a 512-thread
+  // block per SM over single lines 400 threads had nothing to do: 720 points along v1, 512 lines, double-float 54 us and
+  // 33 in the tiled kernel, 29 so; native FP64 600 points 62, 47 and 40)
+  const int most = g->nt;
+  if (!nt && (lines + w - 1) / w > GEN_SMS)
+    while (g->nt > 128 && g->nt / 2 * gen_per_thread<T>() >= w * n) g->nt /= 2;
+  // and, with one block per SM, fewer lines where that shortens the last wave (rounds of blocks times lines) and leaves
+  // half of the threads' work: 1080 points along v1, 1024 lines, native FP64 144 us with three (three rounds, the last a
+  // quarter full), 122 in the tiled kernel, 124 with two; 1250 points 160, 148 and 148
+  if (!nt && g->nt == GEN_MAXNT) {
+    auto line_times = [&](int v) { return ((lines + v - 1) / v + GEN_SMS - 1) / GEN_SMS * v; };
+    for (int v = w - 1; v >= 1 && 2 * v * n >= g->nt * gen_per_thread<T>(); --v)
+      if ((v < 8 || v % 4 == 0) && 20 * line_times(v) < 19 * line_times(w)) w = v;
+  }
+  for (;;) {
     g->w = w;
     gen_divisor((uint32_t)w, &g->w_mul, &g->w_sh);
     // row pitches: neighbouring threads of the reading stage in different banks
@@ -348,6 +362,8 @@ bool gen_make(const dmg_fft_pass &p, int64_t lines, int nt, gen_geom *g, int con
     pos += (size_t)w * 8;
     g->smem = (uint32_t)((pos + 15) & ~(size_t)15);
     if (g->smem <= 232448 / (512 / g->nt) - 1024) break;
+    if (g->nt < most) g->nt *= 2;
+    else if (--w < 1) return false;
   }
   return true;
 }
@@ -797,7 +813,7 @@ int launch_gen_group(const dmg_fft_group &in, cudaStream_t s, int *taken) {
     values += (double)gen_lines_of(in.job[j].p, in.job[j].bt) * in.job[j].p.n;
     if (in.job[j].p.gen && gen_make<T>(in.job[j].p, (int64_t)1 << 30, 0, &g) && g.nt > nt) nt = g.nt;
   }
-  const bool full = values >= 304.0 * nt * gen_per_thread<T>();  // (full tiles of all jobs fill the SMs)
+  const bool full = values >= 2.0 * GEN_SMS * nt * gen_per_thread<T>();  // (full tiles of all jobs fill the SMs)
   for (int j = 0; j < in.count; ++j) {
     const dmg_fft_pass &p = in.job[j].p;
     const int64_t n = gen_lines_of(p, in.job[j].bt);

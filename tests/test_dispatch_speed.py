@@ -61,3 +61,11 @@ def test_direct_primes(shape, name, cuda):
 @pytest.mark.parametrize("shape", [(1331, 512), (512, 1331), (143, 1024)], ids=str)
 def test_twiddled_primes(shape, name, cuda):
     _not_slower(cuda, "packed:" + "|".join("local(%d)" % n for n in shape), shape, name)
+
+
+
+@pytest.mark.parametrize("name", list(ARITH))
+@pytest.mark.parametrize("shape", [(720, 512), (600, 512), (1000, 512), (1536, 512), (512, 1280), (1000, 64)], ids=str)
+def test_lines_for_part_of_the_chip(shape, name, cuda):
+    """As many blocks of any-length lines as SMs, or a few times that."""
+    _not_slower(cuda, "packed:" + "|".join("local(%d)" % n for n in shape), shape, name)
