@@ -147,8 +147,10 @@ __host__ __device__ constexpr RegSched reg_table(int kind, int n, bool t, bool i
 // forward n / RL after the last) are as long as the distance of the values
 // that neighbouring slots hold (the plans' larger factor B of n), whose odd
 // pitch then spreads them over the banks.
-__host__ __device__ constexpr RegSched reg_sched(int kind, int n, bool t, bool inv) {
+// lines: the lines per block where not the table's (the results' bits do not depend on them).
+__host__ __device__ constexpr RegSched reg_sched(int kind, int n, bool t, bool inv, int lines = 0) {
   RegSched s = reg_table(kind, n, t, inv);
+  if (lines > 0) s.w = lines;
   // (native FP64 is bound by its pipe: there the odd radix comes first, where it needs no input twiddles)
   if (t && inv && s.ns > 1 && kind != 0) {
     const int first = s.r[0];
@@ -696,9 +698,10 @@ __device__ __forceinline__ int64_t line_address(const dmg_fft_layout &L, int ndi
   return a;
 }
 
-template <typename T, int NF, bool TF, bool INV>
+// LINES: the lines per block (0: the schedule's)
+template <typename T, int NF, bool TF, bool INV, int LINES>
 struct RegShape {
-  static constexpr RegSched S = reg_sched(reg_kind<T>(), NF, TF, INV);
+  static constexpr RegSched S = reg_sched(reg_kind<T>(), NF, TF, INV, LINES);
   static constexpr int TL = S.tl, W = S.w, NTH = TL * W;
   static constexpr int ES = (int)sizeof(C2<T>);
   static constexpr int V = 128 / ES;  // values per shared-memory wavefront
@@ -781,9 +784,9 @@ struct RegShape {
 // ---------------------------------------------------------------- the kernel
 
 // (tan: the pass's host-made entries, at the places of the whole table)
-template <typename T, int SIGN, int NF, bool TF, int F>
+template <typename T, int SIGN, int NF, bool TF, int LINES, int F>
 __device__ __forceinline__ void reg_twiddles(const C2<T> *roots, const C2<T> *tan, C2<T> *tws, int tid) {
-  using G = RegShape<T, NF, TF, (SIGN > 0)>;
+  using G = RegShape<T, NF, TF, (SIGN > 0), LINES>;
   if constexpr (F < G::S.ns) {
     constexpr int LP = G::LP(F), R = G::R(F), PJ = G::tw_per_j(F), TS = NF / (LP * R);
     for (int i = tid; i < PJ * LP; i += G::NTH) {
@@ -805,14 +808,14 @@ __device__ __forceinline__ void reg_twiddles(const C2<T> *roots, const C2<T> *ta
       }
       tws[G::template tw_at<F>(e, j)] = root_at<T, SIGN>(roots, idx % NF);
     }
-    reg_twiddles<T, SIGN, NF, TF, F + 1>(roots, tan, tws, tid);
+    reg_twiddles<T, SIGN, NF, TF, LINES, F + 1>(roots, tan, tws, tid);
   }
 }
 
 // butterflies of stage F on the thread's registers, input twiddles included
-template <typename T, int SIGN, int NF, bool TF, int F>
+template <typename T, int SIGN, int NF, bool TF, int LINES, int F>
 __device__ __forceinline__ void reg_butterfly(C2<T> *a, const C2<T> *tws, int j) {
-  using G = RegShape<T, NF, TF, (SIGN > 0)>;
+  using G = RegShape<T, NF, TF, (SIGN > 0), LINES>;
   constexpr int R = G::R(F), LP = G::LP(F);
   const C2<T> *tw = tws + G::template tw_at<F>(0, j);
   if constexpr (G::tan(F)) {
@@ -856,10 +859,10 @@ __device__ __forceinline__ void reg_butterfly(C2<T> *a, const C2<T> *tws, int j)
 // after_write: called once the first exchange's values are written.
 // bx: the thread's first buffer position (its line's).  STEP: distance of
 // neighbouring positions of a line (W along v1, 1 along t).
-template <typename T, int SIGN, int NF, bool TF, int F, typename Then>
+template <typename T, int SIGN, int NF, bool TF, int LINES, int F, typename Then>
 __device__ __forceinline__ void reg_exchange(const C2<T> *src, C2<T> *bx, const C2<T> *tws, int bl, C2<T> *out,
                                              Then &&after_write) {
-  using G = RegShape<T, NF, TF, (SIGN > 0)>;
+  using G = RegShape<T, NF, TF, (SIGN > 0), LINES>;
   constexpr int STEP = TF ? 1 : G::W;
   constexpr int P = G::pitch(F - 1);
   // write stage F - 1's results
@@ -893,10 +896,10 @@ __device__ __forceinline__ void reg_exchange(const C2<T> *src, C2<T> *bx, const 
 #pragma unroll
   for (int tr = 0; tr < TR; ++tr) {
     const int b = bl + tr * G::TL;
-    if (NB % G::TL == 0 || b < NB) reg_butterfly<T, SIGN, NF, TF, F>(a + tr * R, tws, b / M);
+    if (NB % G::TL == 0 || b < NB) reg_butterfly<T, SIGN, NF, TF, LINES, F>(a + tr * R, tws, b / M);
   }
   if constexpr (F + 1 < G::S.ns) {
-    reg_exchange<T, SIGN, NF, TF, F + 1>(a, bx, tws, bl, out, after_write);
+    reg_exchange<T, SIGN, NF, TF, LINES, F + 1>(a, bx, tws, bl, out, after_write);
   } else {
 #pragma unroll
     for (int i = 0; i < TR * R; ++i) out[i] = a[i];
@@ -946,11 +949,11 @@ __device__ __forceinline__ void reg_unconvert(C2<T> &v, int sexp) {
 // Ask L2 for the values of a tile (the block's next one), a 128-byte line of
 // memory per request where the lines (along v1) or the values of a line
 // (along t) are contiguous; a hint only.
-template <typename T, int SIGN, int NF, bool TF>
+template <typename T, int SIGN, int NF, bool TF, int LINES>
 __device__ __forceinline__ void reg_prefetch(const dmg_fft_pass &p, const dmg_fft_batch &bt, const reg_lines &lines,
                                              uint32_t tile, uint32_t ntiles, const int32_t *tin, const int2 *sin,
                                              bool slot_in, int tid, int l, int bl) {
-  using G = RegShape<T, NF, TF, (SIGN > 0)>;
+  using G = RegShape<T, NF, TF, (SIGN > 0), LINES>;
   constexpr int PER = 128 / G::ES;                        // values per request
   constexpr int CH = G::W > PER ? (G::W + PER - 1) / PER : 1;  // requests per row of lines
   if (tile >= ntiles) return;
@@ -968,11 +971,11 @@ __device__ __forceinline__ void reg_prefetch(const dmg_fft_pass &p, const dmg_ff
   }
 }
 
-template <typename T, int SIGN, int NF, bool TF>
-__global__ void __launch_bounds__(RegShape<T, NF, TF, (SIGN > 0)>::NTH, RegShape<T, NF, TF, (SIGN > 0)>::S.minb)
+template <typename T, int SIGN, int NF, bool TF, int LINES>
+__global__ void __launch_bounds__(RegShape<T, NF, TF, (SIGN > 0), LINES>::NTH, RegShape<T, NF, TF, (SIGN > 0), LINES>::S.minb)
     fft_reg_kernel(const __grid_constant__ dmg_fft_pass p, const __grid_constant__ dmg_fft_batch bt,
                    const __grid_constant__ reg_lines lines) {
-  using G = RegShape<T, NF, TF, (SIGN > 0)>;
+  using G = RegShape<T, NF, TF, (SIGN > 0), LINES>;
   constexpr int TL = G::TL, W = G::W, NTH = G::NTH, ES = G::ES, NS = G::S.ns;
   constexpr bool DFT = std::is_same<T, df>::value;
   // (constants: device code must not evaluate the schedule's functions, whose table is a host object)
@@ -990,7 +993,7 @@ __global__ void __launch_bounds__(RegShape<T, NF, TF, (SIGN > 0)>::NTH, RegShape
   const int tid = threadIdx.x;
   const bool slot_in = TF && SIGN > 0 && p.perm_in, slot_out = TF && SIGN < 0 && p.perm_out;
 
-  reg_twiddles<T, SIGN, NF, TF, 1>(reinterpret_cast<const C2<T> *>(p.roots), reinterpret_cast<const C2<T> *>(p.tan), tws, tid);
+  reg_twiddles<T, SIGN, NF, TF, LINES, 1>(reinterpret_cast<const C2<T> *>(p.roots), reinterpret_cast<const C2<T> *>(p.tan), tws, tid);
   {
     const int d0 = p.kdim[0], m0 = p.kisz[0] ? p.A[d0] : 1;
     const int64_t *ti = p.in.tab[d0], *to = p.out.tab[d0];
@@ -1157,7 +1160,7 @@ __global__ void __launch_bounds__(RegShape<T, NF, TF, (SIGN > 0)>::NTH, RegShape
 #pragma unroll
       for (int i = 0; i < TR1 * R1; ++i) a[i] = C2<T>{};
     }
-    if constexpr (G::S.ahead == AHEAD_L2) reg_prefetch<T, SIGN, NF, TF>(p, bt, lines, tile + gridDim.x, ntiles, tin, sin, slot_in, tid, l, bl);
+    if constexpr (G::S.ahead == AHEAD_L2) reg_prefetch<T, SIGN, NF, TF, LINES>(p, bt, lines, tile + gridDim.x, ntiles, tin, sin, slot_in, tid, l, bl);
     if (in64) {
 #pragma unroll
       for (int i = 0; i < TR1 * R1; ++i) reg_convert<T>(a[i], sexp);
@@ -1176,7 +1179,7 @@ __global__ void __launch_bounds__(RegShape<T, NF, TF, (SIGN > 0)>::NTH, RegShape
 #pragma unroll
     for (int tr = 0; tr < TR1; ++tr) {
       const int b = bl + tr * TL;
-      if (NB1 % TL == 0 || b < NB1) reg_butterfly<T, SIGN, NF, TF, 0>(a + tr * R1, tws, 0);
+      if (NB1 % TL == 0 || b < NB1) reg_butterfly<T, SIGN, NF, TF, LINES, 0>(a + tr * R1, tws, 0);
     }
 
     // ---- the other stages ----
@@ -1184,7 +1187,7 @@ __global__ void __launch_bounds__(RegShape<T, NF, TF, (SIGN > 0)>::NTH, RegShape
     C2<T> y[TRL * RL];
     // (the staging area and, in slot order, the line pointers have been read by the exchange's barriers)
     if (COPY && TF && slot_in && bl == 0) lptr[l] = source_of(tile + gridDim.x);
-    reg_exchange<T, SIGN, NF, TF, 1>(a, bx, tws, bl, y, [&]() {
+    reg_exchange<T, SIGN, NF, TF, LINES, 1>(a, bx, tws, bl, y, [&]() {
       if constexpr (COPY) start_copies(tile + gridDim.x);
     });
     if (SIGN < 0 && p.twiddle == 1 && act && ytw) {
@@ -1253,16 +1256,16 @@ __global__ void __launch_bounds__(RegShape<T, NF, TF, (SIGN > 0)>::NTH, RegShape
 
 // ---------------------------------------------------------------- launch
 
-template <typename T, int SIGN, int NF, bool TF>
+template <typename T, int SIGN, int NF, bool TF, int LINES = 0>
 int launch_reg_k(const dmg_fft_pass &p, const dmg_fft_batch &bt, reg_lines lines, cudaStream_t s) {
-  using G = RegShape<T, NF, TF, (SIGN > 0)>;
+  using G = RegShape<T, NF, TF, (SIGN > 0), LINES>;
   constexpr size_t smem = G::smem();
   static_assert((smem + 1024) * G::S.minb <= 233472, "shared memory of the resident blocks");
   // offsets made for other radices are no use here: the kernel reads its tables instead
   if (lines.rows.r_in != G::S.r[0]) lines.rows.sum_in = 0;
   if (lines.rows.r_out != G::S.r[G::S.ns - 1]) lines.rows.sum_out = 0;
   if (std::is_same<T, double>::value && !p.tan) return dmg_error(DMG_ERR_ARG, "fft pass: no twiddle table");
-  auto k = fft_reg_kernel<T, SIGN, NF, TF>;
+  auto k = fft_reg_kernel<T, SIGN, NF, TF, LINES>;
   int dev = 0, nsm = 0, per_sm = 0;
   cudaError_t es = allow_smem(k, smem);
   if (es == cudaSuccess) es = resident_blocks(k, G::NTH, smem, &per_sm);
@@ -1313,6 +1316,13 @@ inline reg_lines reg_lines_of(const dmg_fft_pass &p, const dmg_fft_batch &bt) {
   return g;
 }
 
+inline uint32_t sm_count() {
+  int dev = 0, nsm = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  return (uint32_t)nsm;
+}
+
 template <typename T, int SIGN, bool TF>
 int launch_reg_form(const dmg_fft_pass &p, const dmg_fft_batch &bt, cudaStream_t s) {
   const reg_lines g = reg_lines_of(p, bt);
@@ -1331,7 +1341,12 @@ int launch_reg_form(const dmg_fft_pass &p, const dmg_fft_batch &bt, cudaStream_t
     case 384: return launch_reg_k<T, SIGN, 384, TF>(p, bt, g, s);
     case 480: return launch_reg_k<T, SIGN, 480, TF>(p, bt, g, s);
     case 512: return launch_reg_k<T, SIGN, 512, TF>(p, bt, g, s);
-    case 1024: return launch_reg_k<T, SIGN, 1024, TF>(p, bt, g, s);
+    case 1024:
+      // Few lines in 16-byte values: one to a block, so that each has an SM (or half of one) to itself instead of
+      // sharing it with three (64 lines, native FP64, 38 -> 27 us, 25 in the tiled kernel; double-float 22 -> 20).
+      if constexpr (sizeof(C2<T>) == 16)
+        if (g.total <= 2 * sm_count()) return launch_reg_k<T, SIGN, 1024, TF, 1>(p, bt, g, s);
+      return launch_reg_k<T, SIGN, 1024, TF>(p, bt, g, s);
     case 2048:
       if constexpr (std::is_same<T, float>::value) return launch_reg_k<T, SIGN, 2048, TF>(p, bt, g, s);
     default: return dmg_error(DMG_ERR_ARG, "fft pass: no register schedule for length %d", p.n);

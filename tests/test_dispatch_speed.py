@@ -69,3 +69,10 @@ def test_twiddled_primes(shape, name, cuda):
 def test_lines_for_part_of_the_chip(shape, name, cuda):
     """As many blocks of any-length lines as SMs, or a few times that."""
     _not_slower(cuda, "packed:" + "|".join("local(%d)" % n for n in shape), shape, name)
+
+
+
+@pytest.mark.parametrize("name", list(ARITH))
+@pytest.mark.parametrize("shape", [(7, 1024), (1024, 64), (128, 1024), (1024, 300)], ids=str)
+def test_few_long_lines(shape, name, cuda):
+    _not_slower(cuda, "packed:" + "|".join("local(%d)" % n for n in shape), shape, name)
