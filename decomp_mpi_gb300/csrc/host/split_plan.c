@@ -509,6 +509,13 @@ static int line_offsets32(const fft_layout *l, const struct dmg_fft_pass *p) {
   return 1;
 }
 
+/* the lines of a pass over one array */
+static int64_t pass_lines(const struct dmg_split_impl *im, const struct dmg_fft_pass *p) {
+  int64_t values = 1;
+  for (int d = 0; d < im->ndim; ++d) values *= im->L[d];
+  return values / p->n;
+}
+
 /* The form in which a pass runs with its lines in registers: along t or
  * along v1, whichever is fastest in memory on both sides.  Radix schedules
  * of the caller's, ranked sides, different fastest axes and lengths without
@@ -549,16 +556,19 @@ static int gen_side(const fft_layout *l, const struct dmg_fft_pass *p, int32_t *
  *   where both sides are ranked: 256 points with a ranked output 429 / 498,
  *   different fastest axes 367 / 500, 16 points along t 254 / 341 (both sides
  *   ranked 590 / 491, 8 points 731 / 441; without conversions 304 / 233);
- * - native FP64 from 128 points with different fastest axes or one ranked
- *   side: 711 / 752, 742 / 777 (64 points 730 / 668, both ranked 882 / 775);
- * - FP32 16-point lines along t: 133 / 164. */
+ * - native FP64 from 128 points: different fastest axes or one ranked side
+ *   711 / 752, 742 / 777, both ranked 870 / 910 (256 points; 128 within 3 %),
+ *   but not 64 points (730 / 668); 2048 points, 1024 lines, along v1
+ *   168 / 215, along t 182 / 215, while 64 lines are 41 / 36 along t and the
+ *   same along v1: there every line has an SM to itself in both;
+ * - FP32 16-point lines along t: 133 / 164, and one tile of up to 16 of them
+ *   along v1 (10.7 / 13.0: the pass along t leaves its instructions behind). */
 static int tiled_faster(const struct dmg_split_impl *im, const struct dmg_fft_pass *p, const fft_layout *li,
                         const fft_layout *lo, int converts) {
   if (p->radix_runtime || !dmg_fft_fixed_length(p->n)) return 0;
-  const int mixed = p->load_order[0] != p->store_order[0];
   if (im->arith == DMG_ARITH_DF) return converts && p->n != 8 && !(li->ranked && lo->ranked);
-  if (im->arith == DMG_ARITH_FP64) return p->n >= 128 && (li->ranked || lo->ranked ? !(li->ranked && lo->ranked) : mixed);
-  return p->n == 16 && p->load_order[0] == 0 && p->store_order[0] == 0;
+  if (im->arith == DMG_ARITH_FP64) return p->n >= 128 && (p->n < 2048 || pass_lines(im, p) > 152);
+  return p->n == 16 && ((p->load_order[0] == 0 && p->store_order[0] == 0) || pass_lines(im, p) <= 16);
 }
 
 /* Passes that have no compile-time register form: lengths without a

@@ -76,3 +76,12 @@ def test_lines_for_part_of_the_chip(shape, name, cuda):
 @pytest.mark.parametrize("shape", [(7, 1024), (1024, 64), (128, 1024), (1024, 300)], ids=str)
 def test_few_long_lines(shape, name, cuda):
     _not_slower(cuda, "packed:" + "|".join("local(%d)" % n for n in shape), shape, name)
+
+
+
+@pytest.mark.parametrize("name", list(ARITH))
+@pytest.mark.parametrize("spec,shape", [("packed:local(2048)|local(1024)", (2048, 1024)),
+                                        ("packed:local(512)|local(2048)", (512, 2048)),
+                                        ("packed:local(2048)|local(64)", (2048, 64))], ids=lambda v: str(v)[:40])
+def test_lengths_without_a_schedule(spec, shape, name, cuda):
+    _not_slower(cuda, spec, shape, name)
