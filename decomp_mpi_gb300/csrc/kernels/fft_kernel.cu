@@ -121,10 +121,12 @@ extern "C" int dmg_fft_tan_entries(int n, int reg, int sign, double *out) {
   const RegSched s = reg_sched(0, n, reg == DMG_FFT_REG_T, sign > 0);
   int at = 0, lp = 1;
   for (int f = 0; f < s.ns; ++f) {
-    // (as RegShape<double>::tw_per_j; the other stages' entries come from the roots)
-    const int r = s.r[f], per = f == 0 ? 0 : r == 4 || r == 8 ? r : is_pow2(r) ? fma_entries(r) : r - 1;
-    if (out && f > 0 && (r == 4 || r == 8)) tan_table(r, lp, sign, out + 2 * (size_t)at);
-    at += per * lp;
+    // (as RegShape<double>::tw_per_j: the twiddled stages' radices are 4 and 8)
+    const int r = s.r[f];
+    if (f > 0) {
+      if (out) tan_table(r, lp, sign, out + 2 * (size_t)at);
+      at += r * lp;
+    }
     lp *= r;
   }
   return at;

@@ -460,16 +460,13 @@ __device__ __forceinline__ void rdft(C2<T> *a) {
   }
 }
 
-// Native FP64, power-of-two radix R: every layer as radix-2 butterflies
-// y0 = a + t b, y1 = 2 a - y0 (six FMAs; four additions where t is a quarter
-// turn), the stage's input twiddles w^q included.  With n values x_q whose
-// factors are u^q (u = w W_R^e), the even outputs are the n/2 values
-// x_q + u^{n/2} x_{q+n/2} with factors u^q, the odd ones their differences
-// with factors (u W_n)^q; level d so needs w^{R / 2^{d+1}} W_{2^{d+1}}^e for
-// e < 2^d, the upper half of them a quarter turn from the lower.  tw: those
-// entries, [w^{R/2}], [w^{R/4}], [w^{R/8}, w^{R/8} W_8], ...  Outputs in
-// bit-reversed places.
-__host__ __device__ constexpr int fma_entries(int R) { return R <= 2 ? R - 1 : R / 2; }
+// Native FP64, power-of-two radix R without input twiddles (a first stage):
+// every layer as radix-2 butterflies.  The even outputs of n values x_q are
+// the transform of the sums x_q + x_{q+n/2}, the odd ones that of their
+// differences with factors W_n^q; a node at depth d, reached by the choices
+// in e, so adds its second half times W_{2^{d+1}}^e (y0 = a + t b,
+// y1 = 2 a - y0: six FMAs; four additions where t is a quarter turn).
+// Outputs in bit-reversed places.
 __host__ __device__ constexpr int bit_reverse(int k, int R) {
   int r = 0;
   for (int b = 1; b < R; b <<= 1) {
@@ -478,8 +475,6 @@ __host__ __device__ constexpr int bit_reverse(int k, int R) {
   }
   return r;
 }
-// level d, e in the lower half (e < 2^{d-1}, or d = 0)
-__host__ __device__ constexpr int fma_entry(int d, int e) { return d == 0 ? 0 : (1 << (d - 1)) + e; }
 
 template <int SIGN>
 __device__ __forceinline__ void bfly_plain(double2 &a, double2 &b) {
@@ -493,22 +488,15 @@ __device__ __forceinline__ void bfly_plain_rot(double2 &a, double2 &b) {
   b = sub_rot<double, SIGN>(a, b);
   a = t;
 }
-// TW: with input twiddles (else w = 1); N values at a, level D, twiddle exponent E
-template <int SIGN, int R, bool TW, int N, int D, int E>
-__device__ __forceinline__ void fma_node(double2 *a, const double2 *tw) {
+// N values at a, depth D, twiddle exponent E
+template <int SIGN, int R, int N, int D, int E>
+__device__ __forceinline__ void fma_node(double2 *a) {
   if constexpr (N > 1) {
     constexpr int H = N / 2;
     constexpr int HALF = D > 0 ? 1 << (D - 1) : 1;  // e and e + HALF differ by a quarter turn
     constexpr int EL = D > 0 ? E % HALF : 0;
     constexpr bool ROT = D > 0 && E >= HALF;
-    if constexpr (TW) {
-      const double2 t = tw[fma_entry(D, EL)];
-#pragma unroll
-      for (int q = 0; q < H; ++q) {
-        if constexpr (ROT) bfly_tw_rot<SIGN>(a[q], a[q + H], t.x, t.y);
-        else bfly_tw<SIGN>(a[q], a[q + H], t.x, t.y);
-      }
-    } else if constexpr (EL == 0) {
+    if constexpr (EL == 0) {
 #pragma unroll
       for (int q = 0; q < H; ++q) {
         if constexpr (ROT) bfly_plain_rot<SIGN>(a[q], a[q + H]);
@@ -532,8 +520,8 @@ __device__ __forceinline__ void fma_node(double2 *a, const double2 *tw) {
 #pragma unroll
       for (int q = 0; q < H; ++q) bfly_tw<SIGN>(a[q], a[q + H], re, im);
     }
-    fma_node<SIGN, R, TW, H, D + 1, E>(a, tw);
-    fma_node<SIGN, R, TW, H, D + 1, E + (1 << D)>(a + H, tw);
+    fma_node<SIGN, R, H, D + 1, E>(a);
+    fma_node<SIGN, R, H, D + 1, E + (1 << D)>(a + H);
   }
 }
 
@@ -745,11 +733,15 @@ struct RegShape {
   }
   static constexpr size_t buf_bytes() { return (size_t)W * (TF ? line_pitch() : line_values()) * ES; }
   // twiddle table entries per j of stage f
-  static constexpr bool tan(int f) { return std::is_same<T, double>::value && f > 0 && (S.r[f] == 4 || S.r[f] == 8); }
-  static constexpr bool fma(int f) { return std::is_same<T, double>::value && is_pow2(S.r[f]) && S.r[f] <= 32; }
-  static constexpr int tw_per_j(int f) {
-    return f == 0 ? 0 : tan(f) ? S.r[f] : fma(f) ? fma_entries(S.r[f]) : S.r[f] - 1;
+  static constexpr bool tan(int f) { return std::is_same<T, double>::value && f > 0; }
+  static constexpr bool tan_radices() {
+    for (int f = 1; f < S.ns; ++f)
+      if (tan(f) && S.r[f] != 4 && S.r[f] != 8) return false;
+    return true;
   }
+  static_assert(tan_radices(), "native FP64: the twiddled stages have radix 4 or 8");
+  static constexpr bool fma(int f) { return std::is_same<T, double>::value && f == 0 && is_pow2(S.r[f]) && S.r[f] <= 32; }
+  static constexpr int tw_per_j(int f) { return f == 0 ? 0 : tan(f) ? S.r[f] : S.r[f] - 1; }
   // (8-byte entries lie in pairs, so that one 16-byte read gives a thread two)
   static constexpr int tw_rows(int f) { return ES == 8 ? (tw_per_j(f) + 1) & ~1 : tw_per_j(f); }
   static constexpr int tw_base(int f) { return f <= 1 ? 0 : tw_base(f - 1) + tw_rows(f - 1) * LP(f - 1); }
@@ -770,11 +762,8 @@ struct RegShape {
     return al16(tout_off() + (size_t)NF * (TF && !INV ? 8 : 4));
   }
   // AHEAD_COPY: the next tile's values, [place in the thread][thread]
-  static constexpr int slots_per_pass() { return NTH >= NF ? 1 : (NF + NTH - 1) / NTH; }
-  static constexpr int lines_per_pass() { return NTH >= NF ? NTH / NF : 1; }
-  static constexpr int stage_values() {
-    return cmax(TR(0) * S.r[0], TF && INV ? (W + lines_per_pass() - 1) / lines_per_pass() * slots_per_pass() : 0);
-  }
+  static_assert(!TF || S.ahead != AHEAD_COPY, "copies ahead are written for the form along v1");
+  static constexpr int stage_values() { return TR(0) * S.r[0]; }
   static constexpr size_t stage_off() { return al16(ptr_off() + (TF ? (size_t)W * 8 : 0)); }
   static constexpr size_t smem() {
     return stage_off() + (S.ahead == AHEAD_COPY ? al16((size_t)stage_values() * NTH * ES) : 0);
@@ -796,17 +785,7 @@ __device__ __forceinline__ void reg_twiddles(const C2<T> *roots, const C2<T> *ta
         tws[at] = __ldg(tan + at);
         continue;
       }
-      int idx;
-      if constexpr (G::fma(F)) {
-        // level d, exponent e - 2^{d-1}: w^{R / 2^{d+1}} W_{2^{d+1}}^e
-        int d = 0;
-        while (d > 0 ? (e >> d) != 0 : e > 0) ++d;
-        const int x = d == 0 ? 0 : e - (1 << (d - 1));
-        idx = j * TS * (R >> (d + 1)) + x * (NF >> (d + 1));
-      } else {
-        idx = (e + 1) * j * TS;
-      }
-      tws[G::template tw_at<F>(e, j)] = root_at<T, SIGN>(roots, idx % NF);
+      tws[G::template tw_at<F>(e, j)] = root_at<T, SIGN>(roots, (e + 1) * j * TS % NF);
     }
     reg_twiddles<T, SIGN, NF, TF, LINES, F + 1>(roots, tan, tws, tid);
   }
@@ -825,14 +804,7 @@ __device__ __forceinline__ void reg_butterfly(C2<T> *a, const C2<T> *tws, int j)
     if constexpr (R == 8) tan_dft8<SIGN>(a, e);
     else tan_dft4<SIGN>(a, e);
   } else if constexpr (G::fma(F)) {
-    if constexpr (F > 0) {
-      double2 t[fma_entries(R)];
-#pragma unroll
-      for (int e = 0; e < fma_entries(R); ++e) t[e] = tw[e * LP];
-      fma_node<SIGN, R, true, R, 0, 0>(a, t);
-    } else {
-      fma_node<SIGN, R, false, R, 0, 0>(a, nullptr);
-    }
+    fma_node<SIGN, R, R, 0, 0>(a);
     C2<T> y[R];
 #pragma unroll
     for (int s = 0; s < R; ++s) y[s] = a[bit_reverse(s, R)];
@@ -1037,19 +1009,7 @@ __global__ void __launch_bounds__(RegShape<T, NF, TF, (SIGN > 0), LINES>::NTH, R
     return static_cast<const unsigned char *>(bt.src[job]) + line_address(p.in, p.ndim, x) * ES;
   };
   auto start_copies = [&](uint32_t tile) {
-    if (TF && slot_in) {
-#pragma unroll
-      for (int i = 0; i < LI; ++i) {
-        const int lc = l0 + i * LS;
-        const unsigned char *lp = l0 < LS && lc < W ? lptr[lc] : nullptr;
-#pragma unroll
-        for (int j = 0; j < J; ++j) {
-          const int s = s0 + j * NTH;
-          if (lp && (NTH >= NF || NF % NTH == 0 || s < NF))
-            copy_async<ES>(stg + (i * J + j) * NTH, lp + (int64_t)sin[s].y * ES);
-        }
-      }
-    } else if (const unsigned char *src = source_of(tile)) {
+    if (const unsigned char *src = source_of(tile)) {
 #pragma unroll
       for (int tr = 0; tr < TR1; ++tr) {
         const int b = bl + tr * TL;
@@ -1069,13 +1029,7 @@ __global__ void __launch_bounds__(RegShape<T, NF, TF, (SIGN > 0), LINES>::NTH, R
     }
     copy_async_commit();
   };
-  if constexpr (COPY) {
-    if (TF && slot_in) {
-      if (bl == 0) lptr[l] = source_of(blockIdx.x);
-      __syncthreads();
-    }
-    start_copies(blockIdx.x);
-  }
+  if constexpr (COPY) start_copies(blockIdx.x);
 
   for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const uint32_t line = tile * W + l;
@@ -1099,24 +1053,18 @@ __global__ void __launch_bounds__(RegShape<T, NF, TF, (SIGN > 0), LINES>::NTH, R
     if (TF && slot_in) {
       // in slot order through shared memory: lanes run along the slots
       C2<T> v[LI * J];
-      if constexpr (COPY) {
+      __syncthreads();  // the buffer and the pointers of the previous tile have been read
+      if (bl == 0) lptr[l] = src;
+      __syncthreads();
 #pragma unroll
-        for (int i = 0; i < LI * J; ++i) v[i] = stg[i * NTH];
-        __syncthreads();  // the buffer and the pointers of the previous tile have been read
-      } else {
-        __syncthreads();
-        if (bl == 0) lptr[l] = src;
-        __syncthreads();
+      for (int i = 0; i < LI; ++i) {
+        const int lc = l0 + i * LS;
+        const unsigned char *lp = l0 < LS && lc < W ? lptr[lc] : nullptr;
 #pragma unroll
-        for (int i = 0; i < LI; ++i) {
-          const int lc = l0 + i * LS;
-          const unsigned char *lp = l0 < LS && lc < W ? lptr[lc] : nullptr;
-#pragma unroll
-          for (int j = 0; j < J; ++j) {
-            const int s = s0 + j * NTH;
-            v[i * J + j] = C2<T>{};
-            if (lp && (NTH >= NF || NF % NTH == 0 || s < NF)) v[i * J + j] = reg_load<T>(lp + (int64_t)sin[s].y * ES);
-          }
+        for (int j = 0; j < J; ++j) {
+          const int s = s0 + j * NTH;
+          v[i * J + j] = C2<T>{};
+          if (lp && (NTH >= NF || NF % NTH == 0 || s < NF)) v[i * J + j] = reg_load<T>(lp + (int64_t)sin[s].y * ES);
         }
       }
 #pragma unroll
@@ -1185,8 +1133,7 @@ __global__ void __launch_bounds__(RegShape<T, NF, TF, (SIGN > 0), LINES>::NTH, R
     // ---- the other stages ----
     constexpr int RL = G::R(NS - 1), LPL = G::LP(NS - 1), NBL = G::NB(NS - 1), TRL = G::TR(NS - 1);
     C2<T> y[TRL * RL];
-    // (the staging area and, in slot order, the line pointers have been read by the exchange's barriers)
-    if (COPY && TF && slot_in && bl == 0) lptr[l] = source_of(tile + gridDim.x);
+    // (the staging area has been read by the exchange's barriers)
     reg_exchange<T, SIGN, NF, TF, LINES, 1>(a, bx, tws, bl, y, [&]() {
       if constexpr (COPY) start_copies(tile + gridDim.x);
     });
