@@ -222,23 +222,30 @@ int dmg_split_group_launches(int count, SplitPlan const *plans, int direction);
 int dmg_split_set_schedule(SplitPlan plan, int schedule);
 /** The schedule in use: DMG_SCHEDULE_LINES or DMG_SCHEDULE_SPLIT. */
 int dmg_split_get_schedule(SplitPlan plan);
-/** Values per pass tile: 0 for the default (4096 for complex64, 2048 for
- * complex128 in double-float, 1024 in native FP64), else a power of two from
- * 64 up to twice that.  Smaller tiles hold fewer lines side by side; larger
- * ones run the FP32 and double-float passes of power-of-two lengths
- * 256...2048 in one 512-thread block per SM (other passes keep the default),
- * so that passes whose lines are strided in memory move longer rows.  Native
- * FP64 passes take at most 1024 values (one line where a line is longer). */
+/** Values per tile of the tiled pass kernel.  0, the default, leaves every
+ * pass its own kernel: lines in registers where the length has a schedule or
+ * the kernel of any length takes the pass, the tiled kernel for the rest
+ * (tiles of 4096 values for complex64, 2048 for complex128 in double-float,
+ * 1024 in native FP64).  Any other value (a power of two from 64 up to twice
+ * those) runs every pass in the tiled kernel with that tile, the default's
+ * sizes among them: that is slower as a rule (1024^3 complex64 forward 26 ms
+ * against 9.9) and meant for comparisons.  Smaller tiles hold fewer lines
+ * side by side; larger ones run the FP32 and double-float passes of
+ * power-of-two lengths 256...2048 in one 512-thread block per SM (other
+ * passes keep the default's size).  Native FP64 passes take at most 1024
+ * values (one line where a line is longer). */
 int dmg_split_set_tile(SplitPlan plan, int values);
-/** The plan's values per tile as set (0: the default, which gives FP32
- * passes whose lines are strided in memory the wide tiles and the others
- * the two-block kernels' tiles). */
+/** The plan's values per tile as set (0: the default, whose tiled passes take
+ * the wide tiles in FP32 where their lines are strided in memory, and the
+ * two-block kernels' tiles otherwise). */
 int dmg_split_get_tile(SplitPlan plan);
 /* Radix schedules of the passes: DMG_RADIX_FIXED runs the compile-time
  * schedules of the lengths that have one (powers of two 8...2048: radix 8
  * stages, 16 as 4 x 4; the 2,3,5-smooth cube sides) and the plan's radices
  * for the others; DMG_RADIX_PLAN8 and DMG_RADIX_PLAN4 run every pass with
- * the plan's radices in the runtime-length kernel, 8s first or 4s first. */
+ * the plan's radices, 8s first or 4s first, in the register kernel of any
+ * length, or in the tiled kernel's runtime stages where that one does not
+ * take the pass (see dmg_split_run_group). */
 #define DMG_RADIX_FIXED 0
 #define DMG_RADIX_PLAN8 1
 #define DMG_RADIX_PLAN4 2
