@@ -22,10 +22,10 @@
 // Measured on one GB300 against the tiled kernel's runtime stages (GB/s of a
 // pass's bytes over 2^27 FP32 or 2^26 other values, along t / along v1):
 // 105 points FP32 680 / 700 -> 2070 / 2680, double-float 520 / 590 -> 975 /
-// 1575, native FP64 223 / 225 -> 536 / 541; 360 points FP32 540 / 810 -> 1600
-// / 1880, native FP64 379 / 409 -> 482 / 494.  180 x 150 x 105 complex128
+// 1575, native FP64 223 / 225 -> 527 / 531; 360 points FP32 540 / 810 -> 1600
+// / 1880, native FP64 379 / 409 -> 464 / 471.  180 x 150 x 105 complex128
 // double-float with uneven blocks 508 -> 267 us; 16 uneven small cubes in one
-// launch per pass, native FP64, 488 -> 354 us.
+// launch per pass, native FP64, 488 -> 346 us.
 #pragma once
 #include "fft_reg.cuh"
 
